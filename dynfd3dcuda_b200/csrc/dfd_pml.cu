@@ -22,7 +22,7 @@
 namespace dfd {
 
 namespace {
-constexpr int PCW = TK;                 // computing warps: one per row of the tile, all nine fields
+constexpr int PCW = 2 * TK;             // computing warps: two per row of the tile (ROLE of pml_node)
 constexpr int PTOT = PCW * 32 + 32;     // plus one copy-issuing warp
 }  // namespace
 
@@ -240,72 +240,53 @@ struct YZFactors {
   float rby, ddy, aly, rbz, ddz, alz;
 };
 
-template <int FX, int FY, int FZ, int IRK>
+// ROLE 0: the momentum equation (fields 0..2), ROLE 1: the constitutive law (fields 3..8).
+// axis contribution of the role's fields and the ADE update of the face, if any
+template <int ROLE, int AX, int IRK>
+__device__ __forceinline__ void pml_axis(const VolArgs& a, const float* dv, float e0, float e1, float e2,
+                                         const NodeMetric& g, float rb, float dd, float al, int face, int own,
+                                         const float* A, int i, int j, int k, float* hv) {
+  constexpr bool X = AX == 0;
+  float D[3];
+  if (ROLE == 0) {
+    role_terms<0, X>(dv, e0, e1, e2, g.lam, g.mu, g.rrho, D);
+#pragma unroll
+    for (int f = 0; f < 3; f++) hv[f] = X ? D[f] * rb : fmaf(D[f], rb, hv[f]);
+    if (face >= 0) role_face<0, AX, IRK>(a, face, face == own, A, i, j, k, rb, dd, al, D, hv);
+  } else {
+    role_terms<3, X>(dv, e0, e1, e2, g.lam, g.mu, g.rrho, D);
+#pragma unroll
+    for (int f = 0; f < 3; f++) hv[f] = X ? D[f] * rb : fmaf(D[f], rb, hv[f]);
+    if (face >= 0) role_face<3, AX, IRK>(a, face, face == own, A, i, j, k, rb, dd, al, D, hv);
+    role_terms<6, X>(dv, e0, e1, e2, g.lam, g.mu, g.rrho, D);
+#pragma unroll
+    for (int f = 0; f < 3; f++) hv[3 + f] = X ? D[f] * rb : fmaf(D[f], rb, hv[3 + f]);
+    if (face >= 0) role_face<6, AX, IRK>(a, face, face == own, A, i, j, k, rb, dd, al, D, hv + 3);
+  }
+}
+template <int ROLE, int FX, int FY, int FZ, int IRK>
 __device__ __forceinline__ void pml_node(const VolArgs& a, int PW, const float* x0, const float* x1, const float* x2,
                                          const float* x3, const float* x4, const float* cur, const NodeMetric& g,
                                          int i, int j, int k, int fx, int fy, int fz, int own, const float* A,
                                          long long q, const float* P, float damp, float rbx, float ddx, float alx,
                                          const YZFactors& yz) {
   const float r = a.rDH;
-  float hv[9], D[9], dv[9];
-  // x
-  {
+  // fields whose derivatives the role needs, and the fields it updates
+  constexpr int G0 = ROLE == 0 ? 3 : 0, NG = ROLE == 0 ? 6 : 3, H0 = ROLE == 0 ? 0 : 3, H1 = ROLE == 0 ? 3 : 9;
+  float hv[9], dv[NG];
 #pragma unroll
-    for (int f = 0; f < 9; f++) {
-      const int o = f * HBOX;
-      dv[f] = d5v<FX>(x0[o], x1[o], x2[o], x3[o], x4[o]) * r;
-    }
-    role_terms<0, true>(dv + 3, g.ex0, g.ex1, g.ex2, g.lam, g.mu, g.rrho, D);
-    role_terms<3, true>(dv, g.ex0, g.ex1, g.ex2, g.lam, g.mu, g.rrho, D + 3);
-    role_terms<6, true>(dv, g.ex0, g.ex1, g.ex2, g.lam, g.mu, g.rrho, D + 6);
-    const float rb = rbx;
-#pragma unroll
-    for (int f = 0; f < 9; f++) hv[f] = D[f] * rb;
-    if (fx >= 0) {
-      const bool st = fx == own;
-      const float dd = ddx, al = alx;
-      role_face<0, 0, IRK>(a, fx, st, A, i, j, k, rb, dd, al, D, hv + 0);
-      role_face<3, 0, IRK>(a, fx, st, A, i, j, k, rb, dd, al, D + 3, hv + 3);
-      role_face<6, 0, IRK>(a, fx, st, A, i, j, k, rb, dd, al, D + 6, hv + 6);
-    }
+  for (int f = 0; f < NG; f++) {
+    const int o = (G0 + f) * HBOX;
+    dv[f] = d5v<FX>(x0[o], x1[o], x2[o], x3[o], x4[o]) * r;
   }
-  // y
-  {
+  pml_axis<ROLE, 0, IRK>(a, dv, g.ex0, g.ex1, g.ex2, g, rbx, ddx, alx, fx, own, A, i, j, k, hv + H0);
 #pragma unroll
-    for (int f = 0; f < 9; f++) dv[f] = d5s<FY, 1>(cur + f * HBOX) * r;
-    role_terms<0, false>(dv + 3, 0.0f, g.ey1, g.ey2, g.lam, g.mu, g.rrho, D);
-    role_terms<3, false>(dv, 0.0f, g.ey1, g.ey2, g.lam, g.mu, g.rrho, D + 3);
-    role_terms<6, false>(dv, 0.0f, g.ey1, g.ey2, g.lam, g.mu, g.rrho, D + 6);
-    const float rb = yz.rby;
+  for (int f = 0; f < NG; f++) dv[f] = d5s<FY, 1>(cur + (G0 + f) * HBOX) * r;
+  pml_axis<ROLE, 1, IRK>(a, dv, 0.0f, g.ey1, g.ey2, g, yz.rby, yz.ddy, yz.aly, fy, own, A, i, j, k, hv + H0);
 #pragma unroll
-    for (int f = 0; f < 9; f++) hv[f] += D[f] * rb;
-    if (fy >= 0) {
-      const bool st = fy == own;
-      const float dd = yz.ddy, al = yz.aly;
-      role_face<0, 1, IRK>(a, fy, st, A, i, j, k, rb, dd, al, D, hv + 0);
-      role_face<3, 1, IRK>(a, fy, st, A, i, j, k, rb, dd, al, D + 3, hv + 3);
-      role_face<6, 1, IRK>(a, fy, st, A, i, j, k, rb, dd, al, D + 6, hv + 6);
-    }
-  }
-  // z
-  {
-#pragma unroll
-    for (int f = 0; f < 9; f++) dv[f] = d5r<FZ>(cur + f * HBOX, PW) * r;
-    role_terms<0, false>(dv + 3, 0.0f, g.ez1, g.ez2, g.lam, g.mu, g.rrho, D);
-    role_terms<3, false>(dv, 0.0f, g.ez1, g.ez2, g.lam, g.mu, g.rrho, D + 3);
-    role_terms<6, false>(dv, 0.0f, g.ez1, g.ez2, g.lam, g.mu, g.rrho, D + 6);
-    const float rb = yz.rbz;
-#pragma unroll
-    for (int f = 0; f < 9; f++) hv[f] += D[f] * rb;
-    if (fz >= 0) {
-      const bool st = fz == own;
-      const float dd = yz.ddz, al = yz.alz;
-      role_face<0, 2, IRK>(a, fz, st, A, i, j, k, rb, dd, al, D, hv + 0);
-      role_face<3, 2, IRK>(a, fz, st, A, i, j, k, rb, dd, al, D + 3, hv + 3);
-      role_face<6, 2, IRK>(a, fz, st, A, i, j, k, rb, dd, al, D + 6, hv + 6);
-    }
-  }
-  rk_tile_store<0, 9, IRK>(a, a.d.nxyz, q, cur, P, hv, damp);
+  for (int f = 0; f < NG; f++) dv[f] = d5r<FZ>(cur + (G0 + f) * HBOX, PW) * r;
+  pml_axis<ROLE, 2, IRK>(a, dv, 0.0f, g.ez1, g.ez2, g, yz.rbz, yz.ddz, yz.alz, fz, own, A, i, j, k, hv + H0);
+  rk_tile_store<H0, H1, IRK>(a, a.d.nxyz, q, cur, P, hv, damp);
 }
 
 // Warp PCW issues the copies; warps 0..PCW-1 compute, one per row of nodes, all nine
@@ -318,7 +299,7 @@ __device__ __forceinline__ void pml_node(const VolArgs& a, int PW, const float* 
 // the nscen scenarios of tab in one launch; mp0, a0, sc0 describe scenario 0 and give the
 // stage's common values.
 template <int FX, int FY, int FZ, int IRK, bool BATCH>
-__global__ void __maxnreg__(168)
+__global__ void __maxnreg__(96)
     volume_pml_kernel(const __grid_constant__ TileMaps mp0, const __grid_constant__ VolArgs a0,
                       const __grid_constant__ TileSched sc0, const TileScen* __restrict__ tab, int nscen, int nunits,
                       int* err, int* sched) {
@@ -442,7 +423,8 @@ __global__ void __maxnreg__(168)
   // strips: the two half-warps take rows two apart (their stencil rows then fall on
   // disjoint shared-memory banks), lane & 15 the column.
   const int hl = lane >> 4, jl = lane & 15;
-  const int srow = (warp >> 1) * 4 + (warp & 1) + 2 * hl;
+  const int role = warp >= TK ? 1 : 0, wrow = warp - role * TK;
+  const int srow = (wrow >> 1) * 4 + (wrow & 1) + 2 * hl;
   Ring wr, pr, qr;
   int sb = 0;
   for (;;) {
@@ -457,7 +439,7 @@ __global__ void __maxnreg__(168)
     const TileSched& sc = BATCH ? ua.sc : sc0;
     const Dims& d = a.d;
     const PmlUnit pu = pml_unit(sc, a, BATCH ? u - ua.unit0 : u);
-    const int row = pu.strip ? srow : warp, col = pu.strip ? jl : lane;
+    const int row = pu.strip ? srow : wrow, col = pu.strip ? jl : lane;
     const int hc = pu.strip ? (row + RZ) * (STRIP + 8) + col + 4 : (row + RZ) * HW + col + 4;
     const int pc = pu.strip ? row * STRIP + col : row * TJ + col;
     const int j = pu.j0 + col, k = pu.k0 + row;
@@ -524,15 +506,27 @@ __global__ void __maxnreg__(168)
         g.lam = Q[side * PB]; g.mu = Q[(side + 1) * PB]; g.rrho = 1.0f / Q[(side + 2) * PB];
         const float damp = a.dampx ? fminf(dx, dyz) : 1.0f;
         const long long q = qyz + (long long)(i + 3) * d.sx;
-        if (pu.strip || pml) {
-          // (strips hold y-slab nodes and the few interior columns beside them)
-          pml_node<FX, FY, FZ, IRK>(a, pu.strip ? STRIP + 8 : HW, x0, x1, x2, x3, x4, cur, g, i, j, k, fx, fy, fz, pu.face,
-                               P + RG::AOFF * PB, q, P, damp, rbx, ddx, alx, yz);
+        // (strips hold y-slab nodes and the few interior columns beside them)
+        const bool ade = pu.strip || pml;
+        const int pw = pu.strip ? STRIP + 8 : HW;
+        const float* A = P + RG::AOFF * PB;
+        float hv[9];
+        if (role == 0) {
+          if (ade) {
+            pml_node<0, FX, FY, FZ, IRK>(a, pw, x0, x1, x2, x3, x4, cur, g, i, j, k, fx, fy, fz, pu.face, A, q, P, damp,
+                                         rbx, ddx, alx, yz);
+          } else {
+            lean_velocity<FX, FY, FZ>(x0, x1, x2, x3, x4, cur, g, a.rDH, hv);
+            rk_tile_store<0, 3, IRK>(a, d.nxyz, q, cur, P, hv, damp);
+          }
         } else {
-          float hv[9];
-          lean_velocity<FX, FY, FZ>(x0, x1, x2, x3, x4, cur, g, a.rDH, hv);
-          lean_stress<FX, FY, FZ>(x0, x1, x2, x3, x4, cur, g, a.rDH, hv);
-          rk_tile_store<0, 9, IRK>(a, d.nxyz, q, cur, P, hv, damp);
+          if (ade) {
+            pml_node<1, FX, FY, FZ, IRK>(a, pw, x0, x1, x2, x3, x4, cur, g, i, j, k, fx, fy, fz, pu.face, A, q, P, damp,
+                                         rbx, ddx, alx, yz);
+          } else {
+            lean_stress<FX, FY, FZ>(x0, x1, x2, x3, x4, cur, g, a.rDH, hv);
+            rk_tile_store<3, 9, IRK>(a, d.nxyz, q, cur, P, hv, damp);
+          }
         }
       }
       __syncwarp();
