@@ -77,56 +77,22 @@ __device__ __forceinline__ void inv3(const float m[3][3], float r[3][3]) {
 
 // Split nodes -> volume at the fault plane: velocity average and stress from the
 // traction matrix [T1 | avg T2 | avg T3] times the inverse metric (transform.cu:310-385).
-__device__ void fault_to_volume(const FaultArgs& a, const float* FW, float* Wdst, int j1, int k1, float damp) {
+// From registers: fw[field][side] the split-node values, t1 the fault traction layer, mq
+// the nine metric components (xi, eta, zeta rows) and the Jacobian of the fault node.
+__device__ __forceinline__ void fault_to_volume(const FaultArgs& a, const float (*fw)[2], const float* t1,
+                                                const float* mq, float* Wdst, int j1, int k1, float damp) {
   const Dims& d = a.d;
-  long long n = d.nxyz, nyz = d.nyz, pf = j1 + (long long)k1 * d.ny;
-  long long q = idx3(d, d.i0, j1, k1);
+  const long long n = d.nxyz, q = idx3(d, d.i0, j1, k1);
   float met[3][3], im[3][3];
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) met[r][c] = a.M[(3 * c + r) * n + q];
-  float rj = 1.0f / a.M[9 * n + q];
+    for (int c = 0; c < 3; c++) met[r][c] = mq[3 * c + r];
+  float rj = 1.0f / mq[9];
   float tr[3][3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    tr[c][0] = a.T1[(c * 7 + 3) * nyz + pf];
-    tr[c][1] = (FW[(3 + c) * 2 * nyz + pf] + FW[(3 + c) * 2 * nyz + nyz + pf]) * 0.5f;
-    tr[c][2] = (FW[(6 + c) * 2 * nyz + pf] + FW[(6 + c) * 2 * nyz + nyz + pf]) * 0.5f;
-  }
-  inv3(met, im);
-  float sg[3][3];
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) sg[r][c] = (tr[r][0] * im[0][c] + tr[r][1] * im[1][c] + tr[r][2] * im[2][c]) * rj;
-#pragma unroll
-  for (int c = 0; c < 3; c++) Wdst[c * n + q] = (FW[c * 2 * nyz + pf] + FW[c * 2 * nyz + nyz + pf]) * 0.5f * damp;
-  Wdst[3 * n + q] = sg[0][0] * damp;
-  Wdst[4 * n + q] = sg[1][1] * damp;
-  Wdst[5 * n + q] = sg[2][2] * damp;
-  Wdst[6 * n + q] = (sg[0][1] + sg[1][0]) * 0.5f * damp;
-  Wdst[7 * n + q] = (sg[0][2] + sg[2][0]) * 0.5f * damp;
-  Wdst[8 * n + q] = (sg[1][2] + sg[2][1]) * 0.5f * damp;
-}
-
-// fault_to_volume with the split-node values of the stage (fw[field][side]) in registers
-// and every load issued before the first store
-__device__ __forceinline__ void fault_to_volume_r(const FaultArgs& a, const float (*fw)[2], float* Wdst, int j1,
-                                                  int k1, float damp) {
-  const Dims& d = a.d;
-  long long n = d.nxyz, nyz = d.nyz, pf = j1 + (long long)k1 * d.ny;
-  long long q = idx3(d, d.i0, j1, k1);
-  float met[3][3], im[3][3];
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) met[r][c] = a.M[(3 * c + r) * n + q];
-  float rj = 1.0f / a.M[9 * n + q];
-  float tr[3][3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    tr[c][0] = a.T1[(c * 7 + 3) * nyz + pf];
+    tr[c][0] = t1[c];
     tr[c][1] = (fw[3 + c][0] + fw[3 + c][1]) * 0.5f;
     tr[c][2] = (fw[6 + c][0] + fw[6 + c][1]) * 0.5f;
   }
@@ -242,28 +208,139 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
   const int j1 = j + 3, k1 = k + 3, km = d.nk - k;
   const long long pf = j1 + (long long)k1 * d.ny;
   const float* FW = a.FWin;
+  const long long qm = idx3(d, d.i0, j1, k1);
+  // ---- every load of the node comes before its first store: the compiler cannot prove
+  // the arrays distinct, and a load behind a store waits a memory round trip of its own
   float s1[3], s2[3], nv[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) { s1[c] = a.vecs1[c * nyz + pf]; s2[c] = a.vecs2[c * nyz + pf]; }
+  const bool ry = a.rupy[q2] % 7, rz = a.rupz[q2] % 7;
+  // split-node values of the stage input, and DyT2 + DzT3 of both sides
+  float fw[9][2], Dyz[3][2];
+#pragma unroll
+  for (int m = 0; m < 2; m++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      fw[c][m] = FW[(c * 2 + m) * nyz + pf];
+      float v2[7], v3[7];
+      const float* t2 = FW + ((3 + c) * 2 + m) * nyz + pf;
+      const float* t3 = FW + ((6 + c) * 2 + m) * nyz + pf;
+#pragma unroll
+      for (int l = 0; l < 7; l++) {
+        v2[l] = t2[l - 3];
+        v3[l] = t3[(long long)(l - 3) * d.ny];
+      }
+      fw[3 + c][m] = v2[3];
+      fw[6 + c][m] = v3[3];
+      if (a.freenode && km <= 3) {
+        // odd image of the traction above the free surface (constant indexes: the line
+        // stays in registers)
+        if (km == 1) {
+          v3[3] = 0.0f; v3[4] = -v3[2]; v3[5] = -v3[1]; v3[6] = -v3[0];
+        } else if (km == 2) {
+          v3[4] = 0.0f; v3[5] = -v3[3]; v3[6] = -v3[2];
+        } else {
+          v3[5] = 0.0f; v3[6] = -v3[4];
+        }
+      }
+      const float dy = (ry ? L2(v2, 3, FY) : L5(v2, 3, FY)) * a.rDH;
+      const float dz = (rz ? L2(v3, 3, FZ) : L5(v3, 3, FZ)) * a.rDH;
+      Dyz[c][m] = dy + dz;
+    }
+  // tractions of the three layers on either side, and the half-cell masses
+  float lay[2][3][3], Mrho[2], rhom[2], jacm[2];
+#pragma unroll
+  for (int m = 0; m < 2; m++) {
+    rhom[m] = a.rhof[m * nyz + pf];
+#pragma unroll
+    for (int l = 1; l <= 3; l++) {
+      const long long q = idx3(d, d.i0 + (2 * m - 1) * l, j1, k1);
+      trac3(a.Win, a.M, n, q, 0, lay[m][l - 1]);
+      jacm[m] = a.M[9 * n + q];  // the i0 -/+ 3 value feeds the half-cell mass (reference quirk)
+    }
+  }
+  float mq[10], fm[3][2], mT1[3];
+#pragma unroll
+  for (int e = 0; e < 10; e++) mq[e] = a.M[e * n + qm];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    fm[c][0] = a.Fm[c * 2 * nyz + pf];
+    fm[c][1] = a.Fm[c * 2 * nyz + nyz + pf];
+    mT1[c] = a.irk == 0 ? a.T1[(c * 7 + 3) * nyz + pf] : a.mT1[c * nyz + pf];
+  }
+  const bool rs = a.friction_type >= 1;
+  float slip0, state0 = 0.0f, tslip0 = 0.0f, tState0 = 0.0f, cslip0 = 0.0f, cState0 = 0.0f;
+  float pa = 0.0f, pb = 0.0f, pL = 0.0f, pVw = 0.0f, peak = 0.0f, pDc = 0.0f, pC0 = 0.0f, state_in = 0.0f;
+  if (a.irk == 0) {
+    slip0 = a.slip[q2];
+    state0 = a.State[q2];
+  } else {
+    slip0 = a.mslip[q2];
+    state0 = a.mState[q2];
+    tslip0 = a.tslip[q2];
+    tState0 = a.tState[q2];
+  }
+  if (a.irk == 3) { cslip0 = a.cslip[q2]; cState0 = a.cState[q2]; }
+  if (rs) {
+    state_in = a.irk == 0 ? state0 : a.State[q2];
+    pa = a.a[q2]; pb = a.b[q2]; pL = a.L[q2];
+    if (a.friction_type != 1) pVw = a.Vw[q2];
+  } else {
+    peak = a.str_peak[q2]; pDc = a.Dc[q2]; pC0 = a.C0[q2];
+  }
+  const int it = *a.it_dev;
+  const double t = a.irk == 0 ? it * a.dDT : (a.irk == 3 ? (it + 1) * a.dDT : (it + 0.5) * a.dDT);
+  const float G = (float)gt_func(t, a.smooth_load_T);
+  float si[3];  // initial stress of the node now
+  if (a.inport_stress == 1) {
+    si[0] = a.T0x[q2] + G * a.dT0x[q2];
+    si[1] = a.T0y[q2] + G * a.dT0y[q2];
+    si[2] = a.T0z[q2] + G * a.dT0z[q2];
+  } else if (!rs) {
+    si[0] = a.sx[q2]; si[1] = a.sy[q2]; si[2] = a.sz[q2];
+  } else {
+    const double y1 = j + a.jg0 - a.NY / 2;
+    const double z1 = a.freenode ? (double)((a.NZ - 1 - k) - (int)(7.5e3 / a.DH)) : (double)(k - a.NZ / 2);
+    const double r = sqrt(y1 * y1 + z1 * z1) * (double)a.DH;
+    const double Fr = r < 3.0e3 ? exp(r * r / (r * r - 9.0e6)) : 0.0;
+    si[0] = -120e6f;
+    si[1] = (float)(-25e6 * Fr * (double)G + -75e6);
+    si[2] = 0.0f;
+  }
+  const float Pf = rs && a.tpP ? a.tpP[q2] : 0.0f;
+  const int t0_flag = a.init_t0_flag[q2];
+
+  // ---- stores of the trial traction's inputs
+  if (rs || a.inport_stress == 1) { a.sx[q2] = si[0]; a.sy[q2] = si[1]; a.sz[q2] = si[2]; }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    if (a.irk == 0) a.mT1[c * nyz + pf] = mT1[c];
+#pragma unroll
+    for (int l = 1; l <= 3; l++) {
+      a.T1[(c * 7 + 3 - l) * nyz + pf] = lay[0][l - 1][c];
+      a.T1[(c * 7 + 3 + l) * nyz + pf] = lay[1][l - 1][c];
+    }
+  }
 
   // ---- state and slip (rk4.cu:833-935)
+  float hs, sl, State = 0.0f;
   {
     float dV[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) dV[c] = FW[c * 2 * nyz + nyz + pf] - FW[c * 2 * nyz + pf];
+    for (int c = 0; c < 3; c++) dV[c] = fw[c][1] - fw[c][0];
     float vs1 = dV[0] * s1[0] + dV[1] * s1[1] + dV[2] * s1[2];
     float vs2 = dV[0] * s2[0] + dV[1] * s2[1] + dV[2] * s2[2];
-    float hs = sqrtf(vs2 * vs2 + vs1 * vs1);
+    hs = sqrtf(vs2 * vs2 + vs1 * vs1);
     a.hslip[q2] = hs;
     float hState = 0.0f;
-    if (a.friction_type >= 1) {
-      double V = fmax((double)hs, 1e-30), st = a.State[q2];
-      double ra = a.a[q2], rb = a.b[q2], rl = a.L[q2];
+    if (rs) {
+      double V = fmax((double)hs, 1e-30), st = state_in;
+      double ra = pa, rb = pb, rl = pL;
       if (a.friction_type == 1) {
         hState = (float)(rb * a.V0 / rl * (exp((a.f0 - st) / rb) - V / a.V0));
       } else {
         double flv = a.f0 - (rb - ra) * log(V / a.V0);
-        double fss = a.fw + (flv - a.fw) / pow(1. + pow(V / (double)a.Vw[q2], 8), 0.125);
+        double fss = a.fw + (flv - a.fw) / pow(1. + pow(V / (double)pVw, 8), 0.125);
         double psiss = ra * (log(sinh(fss / ra)) + log(2. * (a.V0 / V)));
         hState = (float)(-V / rl * (st - psiss));
       }
@@ -273,95 +350,53 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
     // build up over the thousands of steps of a rupture (the reference sums into the value
     // itself, rk4.cu:833-935)
     if (a.irk == 0) {
-      float st0 = a.State[q2], sl0 = a.slip[q2];
-      a.mState[q2] = st0; a.tState[q2] = a.rkb * hState;
-      a.mslip[q2] = sl0; a.tslip[q2] = a.rkb * hs;
+      a.mState[q2] = state0; a.tState[q2] = a.rkb * hState;
+      a.mslip[q2] = slip0; a.tslip[q2] = a.rkb * hs;
     } else if (a.irk < 3) {
-      a.tState[q2] = fmaf(a.rkb, hState, a.tState[q2]);
-      a.tslip[q2] = fmaf(a.rkb, hs, a.tslip[q2]);
+      a.tState[q2] = fmaf(a.rkb, hState, tState0);
+      a.tslip[q2] = fmaf(a.rkb, hs, tslip0);
     }
     if (a.irk == 3) {
-      a.State[q2] = kahan_add(a.mState[q2], fmaf(a.rkb, hState, a.tState[q2]), a.cState + q2);
-      a.slip[q2] = kahan_add(a.mslip[q2], fmaf(a.rkb, hs, a.tslip[q2]), a.cslip + q2);
+      State = kahan_add(state0, fmaf(a.rkb, hState, tState0), &cState0);
+      sl = kahan_add(slip0, fmaf(a.rkb, hs, tslip0), &cslip0);
+      a.cState[q2] = cState0;
+      a.cslip[q2] = cslip0;
     } else {
-      a.State[q2] = fmaf(a.rka, hState, a.mState[q2]);
-      a.slip[q2] = fmaf(a.rka, hs, a.mslip[q2]);
+      State = fmaf(a.rka, hState, state0);
+      sl = fmaf(a.rka, hs, slip0);
     }
+    a.State[q2] = State;
+    a.slip[q2] = sl;
   }
 
-  // ---- trial traction: T1 layers, split-node DyT2/DzT3, residuals of the half cells
-  if (a.irk == 0)
-#pragma unroll
-    for (int c = 0; c < 3; c++) a.mT1[c * nyz + pf] = a.T1[(c * 7 + 3) * nyz + pf];
-  float Mrho[2], R[3][2], jac_last = 1.0f, rho_last = 1.0f;
+  // ---- trial traction: residuals of the half cells
+  float R[3][2];
   const float DH = a.DH, DH2 = DH * DH;
 #pragma unroll
   for (int m = 0; m < 2; m++) {
-    float jac = 1.0f;
-    float rho = a.rhof[m * nyz + pf];
-#pragma unroll
-    for (int l = 1; l <= 3; l++) {
-      int ii = d.i0 + (2 * m - 1) * l;
-      long long q = idx3(d, ii, j1, k1);
-      float t[3];
-      trac3(a.Win, a.M, n, q, 0, t);
-      jac = a.M[9 * n + q];  // the i0 -/+ 3 value feeds the half-cell mass (reference quirk)
-      int lay = 3 + (2 * m - 1) * l;
-#pragma unroll
-      for (int c = 0; c < 3; c++) a.T1[(c * 7 + lay) * nyz + pf] = t[c];
-    }
-    float DyT[3], DzT[3];
-    const bool ry = a.rupy[q2] % 7, rz = a.rupz[q2] % 7;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const float* t2 = FW + (3 + c) * 2 * nyz + m * nyz;
-      DyT[c] = (ry ? G2(t2, pf, 1, FY) : G5(t2, pf, 1, FY)) * a.rDH;
-      float v3[7];
-      const float* t3 = FW + (6 + c) * 2 * nyz + m * nyz;
-#pragma unroll
-      for (int l = 0; l < 7; l++) v3[l] = t3[pf + (long long)(l - 3) * d.ny];
-      if (a.freenode && km <= 3) {
-        v3[km + 2] = 0.0f;
-        for (int l = km + 3; l < 7; l++) v3[l] = -v3[2 * (km + 2) - l];
-      }
-      DzT[c] = (rz ? L2(v3, 3, FZ) : L5(v3, 3, FZ)) * a.rDH;
+      const float r_ = DFD_A1 * lay[m][0][c] + DFD_A2 * lay[m][1][c] + DFD_A3 * lay[m][2][c];
+      R[c][m] = 0.5f * ((2 * m - 1) * r_ + Dyz[c][m] * DH) * DH2;
     }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float* T = a.T1 + c * 7 * nyz + pf;
-      float r_ = m == 0 ? DFD_A1 * T[2 * nyz] + DFD_A2 * T[1 * nyz] + DFD_A3 * T[0]
-                        : DFD_A1 * T[4 * nyz] + DFD_A2 * T[5 * nyz] + DFD_A3 * T[6 * nyz];
-      R[c][m] = 0.5f * ((2 * m - 1) * r_ + (DyT[c] + DzT[c]) * DH) * DH2;
-    }
-    Mrho[m] = 0.5f * jac * rho * DH * DH2;
-    jac_last = jac;
-    rho_last = rho;
+    Mrho[m] = 0.5f * jacm[m] * rhom[m] * DH * DH2;
   }
-  long long qm = idx3(d, d.i0, j1, k1);
+  const float jac_last = jacm[1], rho_last = rhom[1];
 #pragma unroll
-  for (int c = 0; c < 3; c++) nv[c] = a.M[c * n + qm];
+  for (int c = 0; c < 3; c++) nv[c] = mq[c];
   float n0 = sqrtf(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
-  float jacvec = a.M[9 * n + qm] * n0;
+  float jacvec = mq[9] * n0;
 #pragma unroll
   for (int c = 0; c < 3; c++) nv[c] /= n0;
-  const int it = *a.it_dev;
-  double t = a.irk == 0 ? it * a.dDT : (a.irk == 3 ? (it + 1) * a.dDT : (it + 0.5) * a.dDT);
-  float G = (float)gt_func(t, a.smooth_load_T);
   float dV[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) dV[c] = a.Fm[c * 2 * nyz + nyz + pf] - a.Fm[c * 2 * nyz + pf];
+  for (int c = 0; c < 3; c++) dV[c] = fm[c][1] - fm[c][0];
 
   float Tau[3], Tau_n, Vcheck;
   float T1new[3];
   bool from_tau;
   if (a.friction_type == 0) {
     // ---- slip weakening (trial_slipweakening.cu:322-615)
-    if (a.inport_stress == 1) {
-      a.sx[q2] = a.T0x[q2] + G * a.dT0x[q2];
-      a.sy[q2] = a.T0y[q2] + G * a.dT0y[q2];
-      a.sz[q2] = a.T0z[q2] + G * a.dT0z[q2];
-    }
-    float si[3] = {a.sx[q2], a.sy[q2], a.sz[q2]};
     float den = DH2 * (Mrho[0] * DFD_A0P - DFD_A0M * Mrho[1]);
     float TL[3], Ts[3];
 #pragma unroll
@@ -376,9 +411,9 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
     bool change = false;
     float Tau_s;
     if (Trn >= 0.0f) { Tau_n = 0.0f; change = true; } else Tau_n = Trn;
-    float mus = a.str_peak[q2], sl = a.slip[q2], dc = a.Dc[q2];
+    float mus = peak, dc = pDc;
     float fr = sl <= dc ? mus - (mus - a.mu_d) * sl / dc : a.mu_d;
-    float Tau_c = -fr * Tau_n + a.C0[q2];
+    float Tau_c = -fr * Tau_n + pC0;
     if (Ts0 >= Tau_c) { Tau_s = Tau_c; a.flag_rup[q2] = 1; change = true; }
     else { Tau_s = Ts0; a.flag_rup[q2] = 0; }
     if (change) {
@@ -394,7 +429,7 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
       for (int c = 0; c < 3; c++) Tau[c] = TL[c];
     }
     from_tau = change;
-    Vcheck = a.hslip[q2];
+    Vcheck = hs;
   } else {
     // ---- rate and state (trial_ratestate.cu:374-802), FP64
     double Rr[3][2];
@@ -404,19 +439,7 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
       Rr[1][m] = s1[0] * R[0][m] + s1[1] * R[1][m] + s1[2] * R[2][m];
       Rr[2][m] = s2[0] * R[0][m] + s2[1] * R[1][m] + s2[2] * R[2][m];
     }
-    double y1 = j + a.jg0 - a.NY / 2;
-    double z1 = a.freenode ? (double)((a.NZ - 1 - k) - (int)(7.5e3 / a.DH)) : (double)(k - a.NZ / 2);
-    double r = sqrt(y1 * y1 + z1 * z1) * (double)a.DH;
-    double Fr = r < 3.0e3 ? exp(r * r / (r * r - 9.0e6)) : 0.0;
-    a.sx[q2] = -120e6f;
-    a.sy[q2] = (float)(-25e6 * Fr * (double)G + -75e6);
-    a.sz[q2] = 0.0f;
-    if (a.inport_stress == 1) {
-      a.sx[q2] = a.T0x[q2] + G * a.dT0x[q2];
-      a.sy[q2] = a.T0y[q2] + G * a.dT0y[q2];
-      a.sz[q2] = a.T0z[q2] + G * a.dT0z[q2];
-    }
-    double T0[3] = {a.sx[q2], a.sy[q2], a.sz[q2]};
+    double T0[3] = {si[0], si[1], si[2]};
     double T0l[3] = {nv[0] * T0[0] + nv[1] * T0[1] + nv[2] * T0[2], s1[0] * T0[0] + s1[1] * T0[1] + s1[2] * T0[2],
                      s2[0] * T0[0] + s2[1] * T0[1] + s2[2] * T0[2]};
     double dt1 = a.dDT;
@@ -433,10 +456,9 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
     double tn = Tl[0] >= -1e-1 ? -1e-1 : Tl[0];
     // thermal pressurisation: the friction law sees the effective normal stress tn + P at
     // the fault; the traction put back keeps (tn + P) - P (trial_ratestate.cu:636-643, 787-790)
-    const float Pf = a.tpP ? a.tpP[q2] : 0.0f;
     tn += Pf;
     double Vt1 = cc * Tl[1], Vt2 = cc * Tl[2];
-    double ra = a.a[q2], st = a.State[q2];
+    double ra = pa, st = State;
     double coef = cc * ra * fabs(tn);
     double Vtn = sqrt(Vt1 * Vt1 + Vt2 * Vt2);
     double Ttn = sqrt(Tl[1] * Tl[1] + Tl[2] * Tl[2]);
@@ -552,31 +574,31 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
 #pragma unroll
     tn -= Pf;
     for (int c = 0; c < 3; c++) Tau[c] = (float)(tn * nv[c] + ts1 * s1[c] + ts2 * s2[c]);
-    Tau[0] = a.sx[q2];  // the normal-traction perturbation is forced to zero (:797)
+    Tau[0] = si[0];  // the normal-traction perturbation is forced to zero (:797)
     Tau_n = Tau[0] * nv[0] + Tau[1] * nv[1] + Tau[2] * nv[2];
     from_tau = true;
     Vcheck = Vf;
   }
   // ---- store T1 at the fault, its rate, outputs (trial_slipweakening.cu:629-709)
-  float si[3] = {a.sx[q2], a.sy[q2], a.sz[q2]};
-  float vis = a.viscosity * a.DT;
+  float vis = a.viscosity * a.DT, t1c[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     float v = from_tau ? (Tau[c] - si[c]) * jacvec : T1new[c];
-    float hv = (v - a.mT1[c * nyz + pf]) / a.DT;
+    float hv = (v - mT1[c]) / a.DT;
     if (a.irk == 3) a.hT1[c * nyz + pf] = hv;
-    a.T1[(c * 7 + 3) * nyz + pf] = v + vis * hv;
+    t1c[c] = v + vis * hv;
+    a.T1[(c * 7 + 3) * nyz + pf] = t1c[c];
   }
   a.tTs1[q2] = Tau[0] * s1[0] + Tau[1] * s1[1] + Tau[2] * s1[2];
   a.tTs2[q2] = Tau[0] * s2[0] + Tau[1] * s2[1] + Tau[2] * s2[2];
   a.tTn[q2] = Tau_n;
-  if (!a.init_t0_flag[q2] && Vcheck > 1e-3f) {
+  if (!t0_flag && Vcheck > 1e-3f) {
     a.init_t0[q2] = (float)(it * a.dDT);
     a.init_t0_flag[q2] = 1;
     a.flag_rup[q2] = 1;
   }
   // ---- fault plane into the stage input (transform.cu:224-403)
-  fault_to_volume(a, FW, a.Win, j1, k1, 1.0f);
+  fault_to_volume(a, fw, t1c, mq, a.Win, j1, k1, 1.0f);
 }
 
 // stress RHS of a volume node from its velocity gradient (fault_dstrs_f.cu:1213-1248)
@@ -874,6 +896,11 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
   float s1[3], s2[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) { s1[c] = a.vecs1[c * nyz + pf]; s2[c] = a.vecs2[c * nyz + pf]; }
+  float t1c[3], mq[10];
+#pragma unroll
+  for (int c = 0; c < 3; c++) t1c[c] = a.T1[(c * 7 + 3) * nyz + pf];
+#pragma unroll
+  for (int e = 0; e < 10; e++) mq[e] = M[e * n + idx3(d, i0, j1, k1)];
   const float tts1 = a.tTs1[q2], tts2 = a.tTs2[q2], ttn = a.tTn[q2];
   float ts1 = 0.0f, ts2 = 0.0f, tn = 0.0f;
   if (a.irk != 0) { ts1 = a.Ts1[q2]; ts2 = a.Ts2[q2]; tn = a.Tn[q2]; }
@@ -917,7 +944,7 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
     }
   }
   float damp0 = a.dampx ? fminf(a.dampx[i0], dampyz) : 1.0f;
-  fault_to_volume_r(a, wv, a.Wout, j1, k1, damp0);
+  fault_to_volume(a, wv, t1c, mq, a.Wout, j1, k1, damp0);
 }
 
 template <int FY, int FZ>
