@@ -27,6 +27,17 @@ __device__ __forceinline__ float L3(const float* v, int c, int F) {
   return F == 1 ? -DFD_C24_1 * v[c] + DFD_C24_2 * v[c + 1] - DFD_C24_3 * v[c + 2]
                 : DFD_C24_3 * v[c - 2] - DFD_C24_2 * v[c - 1] + DFD_C24_1 * v[c];
 }
+// odd image of a 7-point line of T3 about the free surface km - 1 rows above its centre
+// (km 1..3), with constant indexes so that the line stays in registers
+__device__ __forceinline__ void free_image(float* v, int km) {
+  if (km == 1) {
+    v[3] = 0.0f; v[4] = -v[2]; v[5] = -v[1]; v[6] = -v[0];
+  } else if (km == 2) {
+    v[4] = 0.0f; v[5] = -v[3]; v[6] = -v[2];
+  } else {
+    v[5] = 0.0f; v[6] = -v[4];
+  }
+}
 // strided global versions
 __device__ __forceinline__ float G5(const float* v, long long q, long long s, int F) {
   return F == 1 ? -DFD_C1 * v[q - s] - DFD_C2 * v[q] + DFD_C3 * v[q + s] - DFD_C4 * v[q + 2 * s] + DFD_C5 * v[q + 3 * s]
@@ -40,6 +51,12 @@ __device__ __forceinline__ float G3(const float* v, long long q, long long s, in
                 : DFD_C24_3 * v[q - 2 * s] - DFD_C24_2 * v[q - s] + DFD_C24_1 * v[q];
 }
 
+// the same on the five points of the operator's window (c - 1 .. c + 3, or c - 3 .. c + 1)
+template <int F>
+__device__ __forceinline__ float W5(const float* w) {
+  return F == 1 ? -DFD_C1 * w[0] - DFD_C2 * w[1] + DFD_C3 * w[2] - DFD_C4 * w[3] + DFD_C5 * w[4]
+                : -DFD_C5 * w[0] + DFD_C4 * w[1] - DFD_C3 * w[2] + DFD_C2 * w[3] + DFD_C1 * w[4];
+}
 __device__ __forceinline__ void trac3(const float* W, const float* M, long long n, long long q, int mo, float* t) {
   float e0 = M[mo * n + q], e1 = M[(mo + 1) * n + q], e2 = M[(mo + 2) * n + q], jac = M[9 * n + q];
   float txx = W[3 * n + q], tyy = W[4 * n + q], tzz = W[5 * n + q];
@@ -233,15 +250,7 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
       fw[3 + c][m] = v2[3];
       fw[6 + c][m] = v3[3];
       if (a.freenode && km <= 3) {
-        // odd image of the traction above the free surface (constant indexes: the line
-        // stays in registers)
-        if (km == 1) {
-          v3[3] = 0.0f; v3[4] = -v3[2]; v3[5] = -v3[1]; v3[6] = -v3[0];
-        } else if (km == 2) {
-          v3[4] = 0.0f; v3[5] = -v3[3]; v3[6] = -v3[2];
-        } else {
-          v3[5] = 0.0f; v3[6] = -v3[4];
-        }
+        free_image(v3, km);
       }
       const float dy = (ry ? L2(v2, 3, FY) : L5(v2, 3, FY)) * a.rDH;
       const float dz = (rz ? L2(v3, 3, FZ) : L5(v3, 3, FZ)) * a.rDH;
@@ -601,13 +610,13 @@ __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, flo
   fault_to_volume(a, fw, t1c, mq, a.Win, j1, k1, 1.0f);
 }
 
-// stress RHS of a volume node from its velocity gradient (fault_dstrs_f.cu:1213-1248)
-__device__ __forceinline__ void hooke(const float* M, long long n, long long q, const float* X, const float* Y,
-                                      const float* Z, float* hT) {
-  float lam = M[10 * n + q], mu = M[11 * n + q], l2m = lam + 2.0f * mu;
-  float ex0 = M[q], ex1 = M[n + q], ex2 = M[2 * n + q];
-  float ey0 = M[3 * n + q], ey1 = M[4 * n + q], ey2 = M[5 * n + q];
-  float ez0 = M[6 * n + q], ez1 = M[7 * n + q], ez2 = M[8 * n + q];
+// stress RHS of a volume node from its velocity gradient (fault_dstrs_f.cu:1213-1248);
+// m: the node's metric rows, Jacobian, lambda, mu, rho
+__device__ __forceinline__ void hooke(const float* m, const float* X, const float* Y, const float* Z, float* hT) {
+  float lam = m[10], mu = m[11], l2m = lam + 2.0f * mu;
+  float ex0 = m[0], ex1 = m[1], ex2 = m[2];
+  float ey0 = m[3], ey1 = m[4], ey2 = m[5];
+  float ez0 = m[6], ez1 = m[7], ez2 = m[8];
   hT[0] = l2m * ex0 * X[0] + lam * ex1 * X[1] + lam * ex2 * X[2] + l2m * ey0 * Y[0] + lam * ey1 * Y[1] +
           lam * ey2 * Y[2] + l2m * ez0 * Z[0] + lam * ez1 * Z[1] + lam * ez2 * Z[2];
   hT[1] = lam * ex0 * X[0] + l2m * ex1 * X[1] + lam * ex2 * X[2] + lam * ey0 * Y[0] + l2m * ey1 * Y[1] +
@@ -653,22 +662,38 @@ __device__ __forceinline__ void rk_store9(const FaultArgs& a, long long q, const
   }
 }
 
-template <int FX, int FY, int FZ>
-__device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int by, int part) {
+// Traction planes of a block's 32 x 4 nodes of one off-fault layer, with the halo of the y
+// (T2 = jac eta . sigma) and z (T3 = jac zeta . sigma) operators.
+struct BandTile {
+  float t2[3][4][36], t3[3][8][32];
+};
+
+// T3 of row kk (interior index) of column j into the tile; rows above the free surface
+// hold the odd image of the rows below it
+__device__ __forceinline__ void band_stage_t3(const FaultArgs& a, int i, int j, int kk, float* t) {
   const Dims& d = a.d;
-  int j = bx * blockDim.x + threadIdx.x;
-  int k = by * blockDim.y + threadIdx.y;
-  if (j >= d.nj || k >= d.nk) return;
-  int q2 = j + k * d.nj;
-  if (a.united[q2]) {
+  t[0] = t[1] = t[2] = 0.0f;
+  if (j + 3 >= d.ny || kk + 3 >= d.nz) return;  // beyond what any node's operator reads
+  const bool image = a.freenode && kk > d.nk - 1;
+  trac3(a.Win, a.M, d.nxyz, idx3(d, i, j + 3, (image ? 2 * (d.nk - 1) - kk : kk) + 3), 6, t);
+  if (image) { t[0] = -t[0]; t[1] = -t[1]; t[2] = -t[2]; }
+}
+
+template <int FX, int FY, int FZ>
+__device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int by, int part, BandTile& bt) {
+  const Dims& d = a.d;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int j = bx * 32 + tx, k = by * 4 + ty;
+  const bool inside = j < d.nj && k < d.nk;
+  const int q2 = j + k * d.nj;
+  const bool split = inside && !a.united[q2];
+  if (part == 6 && inside && !split && a.irk == 0) {
     // welded nodes: the RK-weighted outputs run over every node in the reference
     // (rk4.cu:521-569) and are zero there (no trial traction, no split velocity)
-    if (a.irk == 0 && part == 6) {
-      a.Tn[q2] = 0.0f; a.Ts1[q2] = 0.0f; a.Ts2[q2] = 0.0f;
-      a.Vs1[q2] = 0.0f; a.Vs2[q2] = 0.0f; a.hslip[q2] = 0.0f;
-    }
-    return;
+    a.Tn[q2] = 0.0f; a.Ts1[q2] = 0.0f; a.Ts2[q2] = 0.0f;
+    a.Vs1[q2] = 0.0f; a.Vs2[q2] = 0.0f; a.hslip[q2] = 0.0f;
   }
+  if (!__syncthreads_or(split)) return;
   const long long n = d.nxyz, nyz = d.nyz;
   const int j1 = j + 3, k1 = k + 3, km = d.nk - k, i0 = d.i0;
   const long long pf = j1 + (long long)k1 * d.ny;
@@ -676,99 +701,145 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
   const float* FW = a.FWin;
   const float* M = a.M;
   const float r = a.rDH;
-  const bool ry = a.rupy[q2] % 7, rz = a.rupz[q2] % 7;
-  float dampyz = 1.0f;
-  if (a.dampx) dampyz = fminf(a.dampy[j1], a.dampz[k1]);
 
   // ---------------- volume nodes of one of the six off-fault layers (parts 0..5)
   if (part < 6) {
     const int l = part < 3 ? part - 3 : part - 2;
     const int i = i0 + l;
     const long long q = idx3(d, i, j1, k1);
-    // velocity RHS (fault_dvelo.cu:153-254), traction image across the fault
-    int nn = i0 - i;
-    float hv[3];
+    constexpr int RX = FX == 1 ? 1 : 3, RY = FY == 1 ? 1 : 3, RZ = FZ == 1 ? 1 : 3;  // centre of the window
+    // tractions of the tile: each thread its own node and one node of the z halo, sixteen
+    // threads one of the y halo.  A node is evaluated 2.1 times per layer and block instead
+    // of ten times by its neighbours.
+    float m[13];
+    const bool stored = j1 < d.ny && k1 < d.nz;
+    if (stored) {
+#pragma unroll
+      for (int e = 0; e < 13; e++) m[e] = M[e * n + q];
+      const float txx = W[3 * n + q], tyy = W[4 * n + q], tzz = W[5 * n + q];
+      const float txy = W[6 * n + q], txz = W[7 * n + q], tyz = W[8 * n + q];
+      bt.t2[0][ty][tx + RY] = (m[3] * txx + m[4] * txy + m[5] * txz) * m[9];
+      bt.t2[1][ty][tx + RY] = (m[3] * txy + m[4] * tyy + m[5] * tyz) * m[9];
+      bt.t2[2][ty][tx + RY] = (m[3] * txz + m[4] * tyz + m[5] * tzz) * m[9];
+      if (!(a.freenode && k > d.nk - 1)) {
+        bt.t3[0][ty + RZ][tx] = (m[6] * txx + m[7] * txy + m[8] * txz) * m[9];
+        bt.t3[1][ty + RZ][tx] = (m[6] * txy + m[7] * tyy + m[8] * tyz) * m[9];
+        bt.t3[2][ty + RZ][tx] = (m[6] * txz + m[7] * tyz + m[8] * tzz) * m[9];
+      }
+    }
+    float t[3];
+    if (a.freenode && k > d.nk - 1) {
+      band_stage_t3(a, i, j, k, t);
+#pragma unroll
+      for (int c = 0; c < 3; c++) bt.t3[c][ty + RZ][tx] = t[c];
+    }
     {
-      float v1[3][7], v2[3][7], v3[3][7];
+      const int row = ty < RZ ? ty : ty + 4;
+      band_stage_t3(a, i, j, by * 4 + row - RZ, t);
 #pragma unroll
-      for (int s = 0; s < 7; s++) {
-        float t[3];
-        trac3(W, M, n, q + (long long)(s - 3) * d.sx, 0, t);
-        v1[0][s] = t[0]; v1[1][s] = t[1]; v1[2][s] = t[2];
-        trac3(W, M, n, q + (s - 3), 3, t);
-        v2[0][s] = t[0]; v2[1][s] = t[1]; v2[2][s] = t[2];
-        trac3(W, M, n, q + (long long)(s - 3) * d.py, 6, t);
-        v3[0][s] = t[0]; v3[1][s] = t[1]; v3[2][s] = t[2];
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        float* v = v1[c];
-        v[nn + 3] = a.T1[(c * 7 + 3) * nyz + pf];
-        if (nn == 2) v[6] = 2.0f * v[5] - v[4];
-        if (nn == 1) { v[5] = 2.0f * v[4] - v[3]; v[6] = 2.0f * v[4] - v[2]; }
-        if (nn == -1) { v[0] = 2.0f * v[2] - v[4]; v[1] = 2.0f * v[2] - v[3]; }
-        if (nn == -2) v[0] = 2.0f * v[1] - v[2];
-        if (a.freenode && km <= 3) {
-          v3[c][km + 2] = 0.0f;
-          for (int s = km + 3; s < 7; s++) v3[c][s] = -v3[c][2 * (km + 2) - s];
-        }
-      }
-      float rrj = 1.0f / (M[12 * n + q] * M[9 * n + q]);
-#pragma unroll
-      for (int c = 0; c < 3; c++) hv[c] = (L5(v1[c], 3, FX) * r + L5(v2[c], 3, FY) * r + L5(v3[c], 3, FZ) * r) * rrj;
+      for (int c = 0; c < 3; c++) bt.t3[c][row][tx] = t[c];
     }
-    // stress RHS (fault_dstrs_{f,b}.cu, volume columns)
-    float X[3], Y[3], Z[3];
+    if (tx < 4) {
+      const int col = tx < RY ? tx : tx + 32, jc = bx * 32 + col - RY + 3;
+      t[0] = t[1] = t[2] = 0.0f;
+      if (jc < d.ny && k1 < d.nz) trac3(W, M, n, idx3(d, i, jc, k1), 3, t);
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const float* wv = W + c * n;
-      float fm = FW[c * 2 * nyz + pf], fp = FW[c * 2 * nyz + nyz + pf];
-      float x;
-      if (FX == 1) {
-        if (l == 3) x = G5(wv, q, d.sx, 1);
-        else if (l == 2) x = G3(wv, q, d.sx, 1);
-        else if (l == 1) x = wv[q + d.sx] - wv[q];
-        else if (l == -1) x = fm - wv[q];
-        else if (l == -2) x = -DFD_C24_1 * wv[q] + DFD_C24_2 * wv[q + d.sx] - DFD_C24_3 * fm;
-        else x = -DFD_C1 * wv[q - d.sx] - DFD_C2 * wv[q] + DFD_C3 * wv[q + d.sx] - DFD_C4 * wv[q + 2 * d.sx] + DFD_C5 * fm;
-      } else {
-        if (l == -3) x = G5(wv, q, d.sx, -1);
-        else if (l == -2) x = G3(wv, q, d.sx, -1);
-        else if (l == -1) x = wv[q] - wv[q - d.sx];
-        else if (l == 1) x = wv[q] - fp;
-        else if (l == 2) x = DFD_C24_3 * fp - DFD_C24_2 * wv[q - d.sx] + DFD_C24_1 * wv[q];
-        else x = -DFD_C5 * fp + DFD_C4 * wv[q - 2 * d.sx] - DFD_C3 * wv[q - d.sx] + DFD_C2 * wv[q] + DFD_C1 * wv[q + d.sx];
-      }
-      X[c] = x * r;
-      Y[c] = G5(wv, q, 1, FY) * r;
+      for (int c = 0; c < 3; c++) bt.t2[c][ty][col] = t[c];
     }
-    if (a.freenode && km == 1) {
-      const float* mx = a.mVx2Vz + (j1 + (long long)i * d.ny) * 9;
-      const float* my = a.mVy2Vz + (j1 + (long long)i * d.ny) * 9;
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        Z[c] = mx[3 * c] * X[0] + mx[3 * c + 1] * X[1] + mx[3 * c + 2] * X[2] + my[3 * c] * Y[0] + my[3 * c + 1] * Y[1] +
-               my[3 * c + 2] * Y[2];
-    } else {
+    // stress RHS (fault_dstrs_{f,b}.cu, volume columns) and the x line of T1 before the
+    // barrier, so that their loads are in flight with the tile's
+    float hT[6], wx[3][5];
+    if (split) {
+      float X[3], Y[3], Z[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const float* wv = W + c * n;
-        float zz;
-        if (a.freenode && km == 2) zz = G2(wv, q, d.py, FZ);
-        else if (a.freenode && km == 3) zz = G3(wv, q, d.py, FZ);
-        else zz = G5(wv, q, d.py, FZ);
-        Z[c] = zz * r;
+        float fm = FW[c * 2 * nyz + pf], fp = FW[c * 2 * nyz + nyz + pf];
+        float x;
+        if (FX == 1) {
+          if (l == 3) x = G5(wv, q, d.sx, 1);
+          else if (l == 2) x = G3(wv, q, d.sx, 1);
+          else if (l == 1) x = wv[q + d.sx] - wv[q];
+          else if (l == -1) x = fm - wv[q];
+          else if (l == -2) x = -DFD_C24_1 * wv[q] + DFD_C24_2 * wv[q + d.sx] - DFD_C24_3 * fm;
+          else x = -DFD_C1 * wv[q - d.sx] - DFD_C2 * wv[q] + DFD_C3 * wv[q + d.sx] - DFD_C4 * wv[q + 2 * d.sx] + DFD_C5 * fm;
+        } else {
+          if (l == -3) x = G5(wv, q, d.sx, -1);
+          else if (l == -2) x = G3(wv, q, d.sx, -1);
+          else if (l == -1) x = wv[q] - wv[q - d.sx];
+          else if (l == 1) x = wv[q] - fp;
+          else if (l == 2) x = DFD_C24_3 * fp - DFD_C24_2 * wv[q - d.sx] + DFD_C24_1 * wv[q];
+          else x = -DFD_C5 * fp + DFD_C4 * wv[q - 2 * d.sx] - DFD_C3 * wv[q - d.sx] + DFD_C2 * wv[q] + DFD_C1 * wv[q + d.sx];
+        }
+        X[c] = x * r;
+        Y[c] = G5(wv, q, 1, FY) * r;
+      }
+      if (a.freenode && km == 1) {
+        const float* mx = a.mVx2Vz + (j1 + (long long)i * d.ny) * 9;
+        const float* my = a.mVy2Vz + (j1 + (long long)i * d.ny) * 9;
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          Z[c] = mx[3 * c] * X[0] + mx[3 * c + 1] * X[1] + mx[3 * c + 2] * X[2] + my[3 * c] * Y[0] + my[3 * c + 1] * Y[1] +
+                 my[3 * c + 2] * Y[2];
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float* wv = W + c * n;
+          float zz;
+          if (a.freenode && km == 2) zz = G2(wv, q, d.py, FZ);
+          else if (a.freenode && km == 3) zz = G3(wv, q, d.py, FZ);
+          else zz = G5(wv, q, d.py, FZ);
+          Z[c] = zz * r;
+        }
+      }
+      hooke(m, X, Y, Z, hT);
+      // T1 along x: the layers within three of the fault and the fault itself as the node
+      // kernel stored them, across the fault their odd image about the fault traction
+      // (fault_dvelo.cu:153-254), further out from the wavefield
+#pragma unroll
+      for (int s = 0; s < 5; s++) {
+        const int L = l + s - RX;
+        if (L > 3 || L < -3) {
+          trac3(W, M, n, q + (long long)(s - RX) * d.sx, 0, t);
+          wx[0][s] = t[0]; wx[1][s] = t[1]; wx[2][s] = t[2];
+        } else if (L * l >= 0) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) wx[c][s] = a.T1[(c * 7 + 3 + L) * nyz + pf];
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; c++)
+            wx[c][s] = 2.0f * a.T1[(c * 7 + 3) * nyz + pf] - a.T1[(c * 7 + 3 - L) * nyz + pf];
+        }
       }
     }
-    float hT[6];
-    hooke(M, n, q, X, Y, Z, hT);
-    float damp = a.dampx ? fminf(a.dampx[i], dampyz) : 1.0f;
-    const float h9[9] = {hv[0], hv[1], hv[2], hT[0], hT[1], hT[2], hT[3], hT[4], hT[5]};
+    __syncthreads();
+    if (!split) return;
+    // velocity RHS (fault_dvelo.cu:153-254)
+    const float rrj = 1.0f / (m[12] * m[9]);
+    const int top = a.freenode && km <= 3 ? km - 1 + RZ : -1;  // the traction-free row in the z window
+    float h9[9];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      float wy[5], wz[5];
+#pragma unroll
+      for (int s = 0; s < 5; s++) {
+        wy[s] = bt.t2[c][ty][tx + s];
+        wz[s] = s == top ? 0.0f : bt.t3[c][ty + s][tx];
+      }
+      h9[c] = (W5<FX>(wx[c]) * r + W5<FY>(wy) * r + W5<FZ>(wz) * r) * rrj;
+    }
+#pragma unroll
+    for (int c = 0; c < 6; c++) h9[3 + c] = hT[c];
+    float damp = a.dampx ? fminf(a.dampx[i], fminf(a.dampy[j1], a.dampz[k1])) : 1.0f;
     rk_store9(a, q, h9, damp);
+    return;
   }
 
   // ---------------- split nodes (part 6)
-  if (part != 6) return;
+  if (!split) return;
+  const bool ry = a.rupy[q2] % 7, rz = a.rupz[q2] % 7;
+  float dampyz = 1.0f;
+  if (a.dampx) dampyz = fminf(a.dampy[j1], a.dampz[k1]);
   float hF[9][2];
   // velocity RHS on both sides (fault_dvelo.cu:260-385)
 #pragma unroll
@@ -787,8 +858,7 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
       for (int s = 0; s < 7; s++) v3[s] = t3[pf + (long long)(s - 3) * d.ny];
       float dz;
       if (a.freenode && km <= 3) {
-        v3[km + 2] = 0.0f;
-        for (int s = km + 3; s < 7; s++) v3[s] = -v3[2 * (km + 2) - s];
+        free_image(v3, km);
         dz = L5(v3, 3, FZ) * r;
       } else {
         dz = (rz ? L2(v3, 3, FZ) : L5(v3, 3, FZ)) * r;
@@ -958,7 +1028,8 @@ __global__ void __launch_bounds__(128) fault_node_kernel(const __grid_constant__
 // loses to the few spilled values (measured: 3, 4, 5, 6 blocks per SM).
 template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_band_kernel(const __grid_constant__ FaultArgs a) {
-  fault_band_body<FX, FY, FZ>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+  __shared__ BandTile bt;
+  fault_band_body<FX, FY, FZ>(a, blockIdx.x, blockIdx.y, blockIdx.z, bt);
 }
 
 // Batched launches over the scenarios of an ensemble: scenario s owns the blocks
@@ -979,6 +1050,7 @@ template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_band_batch(const FaultArgs* __restrict__ tab, const int* __restrict__ start,
                                                         int n) {
   __shared__ __align__(16) unsigned char raw[sizeof(FaultArgs)];
+  __shared__ BandTile bt;
   FaultArgs* sa = reinterpret_cast<FaultArgs*>(raw);
   int loc;
   const int sc = scenario_of(start, n, blockIdx.x, &loc);
@@ -987,7 +1059,7 @@ __global__ void __launch_bounds__(128, 4) fault_band_batch(const FaultArgs* __re
   const FaultArgs& a = *sa;
   const int gx = (a.d.nj + 31) / 32, gxy = gx * ((a.d.nk + 3) / 4);
   // the scenario's blocks: seven parts of its (32, 4)-block grid
-  fault_band_body<FX, FY, FZ>(a, (loc % gxy) % gx, (loc % gxy) / gx, loc / gxy);
+  fault_band_body<FX, FY, FZ>(a, (loc % gxy) % gx, (loc % gxy) / gx, loc / gxy, bt);
 }
 
 // Thermal pressurisation (thermpress.cu:22-236), once per step before the stages.  Each
