@@ -1073,11 +1073,12 @@ __global__ void __launch_bounds__(128, 4) fault_band_batch(const FaultArgs* __re
 // values are FP32.  Columns are node-major ([q][i]); point 0 of T and P is also written to
 // two (NZ, NY) planes, which the friction law and the outputs read.
 
-// per-node scalars of the scheme (thermpress.cu:150-175), as the reference rounds them
+// per-node scalars of the scheme (thermpress.cu:150-175), as the reference rounds them; the
+// sub-steps multiply by the FP64 reciprocals rdh2 and rfden, formed once per node
 struct TpNode {
   float rate, Tau_n, fr, ahy, dh, dh2, dt;
   int nsub;
-  double fden;
+  double rdh2, rfden;
 };
 __device__ __forceinline__ TpNode tp_node(const TpArgs& a, int q) {
   const float rho_c = 2.7e6f, h = 20e-3f, alpha_th = 1.0e-6f;
@@ -1094,7 +1095,8 @@ __device__ __forceinline__ TpNode tp_node(const TpArgs& a, int q) {
   const float dt0 = (float)(0.1 * (double)t.dh2 / (double)amax);
   t.nsub = (int)(a.DT / dt0) + 1;
   t.dt = (float)((double)a.DT / (double)t.nsub);
-  t.fden = (double)(rho_c * h) * 2.506628274631000;
+  t.rdh2 = 1.0 / (double)t.dh2;
+  t.rfden = 1.0 / ((double)(rho_c * h) * 2.506628274631000);
   return t;
 }
 
@@ -1104,9 +1106,9 @@ __device__ __forceinline__ void tp_point(const TpNode& t, double g, double fac, 
                                          float Pr, float Pl, float* To, float* Po) {
   const float Lamb = 0.1e6f, alpha_th = 1.0e-6f;
   const float omega = (float)(g * fac);
-  const float dT = (float)((double)alpha_th * ((double)Tr - 2.0 * (double)Tc + (double)Tl) / (double)t.dh2 +
+  const float dT = (float)((double)alpha_th * ((double)Tr - 2.0 * (double)Tc + (double)Tl) * t.rdh2 +
                            (double)omega);
-  const float dP = (float)((double)t.ahy * ((double)Pr - 2.0 * (double)Pc + (double)Pl) / (double)t.dh2 +
+  const float dP = (float)((double)t.ahy * ((double)Pr - 2.0 * (double)Pc + (double)Pl) * t.rdh2 +
                            (double)(Lamb * dT));
   *To = fmaf(t.dt, dT, Tc);
   *Po = fmaf(t.dt, dP, Pc);
@@ -1144,7 +1146,7 @@ __global__ void __launch_bounds__(256) thermpress_warp_kernel(const TpArgs a) {
   for (int sub = 0; sub < t.nsub; sub++) {
     const float P0 = __shfl_sync(FULL, P[0], 0);
     const float tau = -t.fr * (t.Tau_n + P0);
-    const double fac = (double)(tau * t.rate) / t.fden;
+    const double fac = (double)(tau * t.rate) * t.rfden;
     float Tn[K], Pn[K];
 #pragma unroll
     for (int m = 0; m < K; m++) {
@@ -1187,7 +1189,7 @@ __global__ void __launch_bounds__(128) thermpress_column_kernel(const TpArgs a) 
   float* P = a.P + (long long)q * n;
   for (int sub = 0; sub < t.nsub; sub++) {
     const float tau = -t.fr * (t.Tau_n + P[0]);
-    const double fac = (double)(tau * t.rate) / t.fden;
+    const double fac = (double)(tau * t.rate) * t.rfden;
     float Tb = 0.0f, Pb = 0.0f;  // old values of point i - 1
     float Tc = T[0], Pc = P[0];  // old values of point i
     for (int i = 0; i < n; i++) {
