@@ -26,9 +26,9 @@ __device__ __forceinline__ float d5(const float* __restrict__ v, long long q, lo
            DFD_C2 * __ldg(v + q) + DFD_C1 * __ldg(v + q + s);
 }
 template <int F>
-__device__ __forceinline__ float d5a(const float* v, int c) {  // on a 7-point register line, centre c
-  if (F == 1) return -DFD_C1 * v[c - 1] - DFD_C2 * v[c] + DFD_C3 * v[c + 1] - DFD_C4 * v[c + 2] + DFD_C5 * v[c + 3];
-  else return -DFD_C5 * v[c - 3] + DFD_C4 * v[c - 2] - DFD_C3 * v[c - 1] + DFD_C2 * v[c] + DFD_C1 * v[c + 1];
+__device__ __forceinline__ float d5w(const float* v) {  // on the five points of the operator's window
+  if (F == 1) return -DFD_C1 * v[0] - DFD_C2 * v[1] + DFD_C3 * v[2] - DFD_C4 * v[3] + DFD_C5 * v[4];
+  else return -DFD_C5 * v[0] + DFD_C4 * v[1] - DFD_C3 * v[2] + DFD_C2 * v[3] + DFD_C1 * v[4];
 }
 
 // traction vector jac * e_axis . sigma at node q
@@ -43,10 +43,9 @@ __device__ __forceinline__ void traction(const float* __restrict__ W, const floa
   t3 = (e0 * txz + e1 * tyz + e2 * tzz) * jac;
 }
 
-// General node update: every boundary treatment (PML faces, free-surface rows and
-// traction image, sponge).  Used for the shell of the domain outside the interior box;
-// TOP = false leaves out the free-surface terms (nodes below the top three rows).
-template <int FX, int FY, int FZ, bool TOP, int IRK>
+// General node update below the free-surface rows: PML faces and sponge.  Used for the
+// shell of the domain outside the plain interior kernel's box.
+template <int FX, int FY, int FZ, int IRK>
 __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, int j, int k) {
   const Dims& d = a.d;
   int i1 = i + 3, j1 = j + 3, k1 = k + 3;
@@ -62,10 +61,6 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
   float h[9], p[9], dv[9], D[9];
 #pragma unroll
   for (int f = 0; f < 9; f++) p[f] = 0.0f;
-  float dxv[3], dyv[3];
-  // free-surface rows (only in the TOP variant; the other boxes lie below them)
-  const bool fs = TOP && a.freenode && k >= d.nk - 3;
-  const bool top = fs && k == d.nk - 1;
   const bool px1 = a.aux[0] && i < d.N, px2 = a.aux[1] && i >= d.ni - d.N;
   const bool py1 = a.aux[2] && j < d.N, py2 = a.aux[3] && j >= d.nj - d.N;
   const bool pz1 = a.aux[4] && k < d.N, pz2 = a.aux[5] && k >= d.nk - d.N;
@@ -74,110 +69,38 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
   // ---- x ----
 #pragma unroll
   for (int f = 0; f < 9; f++) dv[f] = d5<FX>(W + f * n, q, d.sx) * a.rDH;
-  dxv[0] = dv[0]; dxv[1] = dv[1]; dxv[2] = dv[2];
   axis_terms(dv, __ldg(M + q), __ldg(M + n + q), __ldg(M + 2 * n + q), lam, mu, rrho, D);
 #pragma unroll
   for (int f = 0; f < 9; f++) h[f] = D[f] * rb1;
   if (px1 || px2) {
-    float dz[3];
-    if (top) {
-      const float* m = a.mVx2Vz + (j1 + (long long)i1 * d.ny) * 9;
-#pragma unroll
-      for (int r = 0; r < 3; r++) dz[r] = m[3 * r] * dxv[0] + m[3 * r + 1] * dxv[1] + m[3 * r + 2] * dxv[2];
-    }
     const int fc = px1 ? 0 : 1;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
     pml_face<IRK>(a, fc, qa, st, rb1, __ldg(a.Bx + i), __ldg(a.Dpx + i), __ldg(a.Apx + i), D,
-             top ? dz : nullptr, ez0, ez1, ez2, lam, mu, p);
+             nullptr, ez0, ez1, ez2, lam, mu, p);
   }
   // ---- y ----
 #pragma unroll
   for (int f = 0; f < 9; f++) dv[f] = d5<FY>(W + f * n, q, 1) * a.rDH;
-  dyv[0] = dv[0]; dyv[1] = dv[1]; dyv[2] = dv[2];
   axis_terms(dv, __ldg(M + 3 * n + q), __ldg(M + 4 * n + q), __ldg(M + 5 * n + q), lam, mu, rrho, D);
 #pragma unroll
   for (int f = 0; f < 9; f++) h[f] += D[f] * rb2;
   if (py1 || py2) {
-    float dz[3];
-    if (top) {
-      const float* m = a.mVy2Vz + (j1 + (long long)i1 * d.ny) * 9;
-#pragma unroll
-      for (int r = 0; r < 3; r++) dz[r] = m[3 * r] * dyv[0] + m[3 * r + 1] * dyv[1] + m[3 * r + 2] * dyv[2];
-    }
     const int fc = py1 ? 2 : 3;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
     pml_face<IRK>(a, fc, qa, st, rb2, __ldg(a.By + j), __ldg(a.Dpy + j), __ldg(a.Apy + j), D,
-             top ? dz : nullptr, ez0, ez1, ez2, lam, mu, p);
+             nullptr, ez0, ez1, ez2, lam, mu, p);
   }
   // ---- z ----
 #pragma unroll
   for (int f = 0; f < 9; f++) dv[f] = d5<FZ>(W + f * n, q, d.py) * a.rDH;
-  float Dz_plain[9];
-  axis_terms(dv, ez0, ez1, ez2, lam, mu, rrho, Dz_plain);
-#pragma unroll
-  for (int f = 0; f < 9; f++) D[f] = Dz_plain[f];
-  if (fs) {
-    // velocity z-derivatives on the top rows (wave.cu:205-245)
-    float dz[3];
-    if (k == d.nk - 1) {
-      const float* mx = a.mVx2Vz + (j1 + (long long)i1 * d.ny) * 9;
-      const float* my = a.mVy2Vz + (j1 + (long long)i1 * d.ny) * 9;
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-        dz[r] = (mx[3 * r] * dxv[0] + mx[3 * r + 1] * dxv[1] + mx[3 * r + 2] * dxv[2]) +
-                (my[3 * r] * dyv[0] + my[3 * r + 1] * dyv[1] + my[3 * r + 2] * dyv[2]);
-    } else if (k == d.nk - 2) {
-#pragma unroll
-      for (int r = 0; r < 3; r++) {
-        const float* v = W + r * n;
-        dz[r] = (FZ == 1 ? (__ldg(v + q + d.py) - __ldg(v + q)) : (__ldg(v + q) - __ldg(v + q - d.py))) * a.rDH;
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < 3; r++) {
-        const float* v = W + r * n;
-        dz[r] = (FZ == 1 ? (-DFD_C24_1 * __ldg(v + q) + DFD_C24_2 * __ldg(v + q + d.py) - DFD_C24_3 * __ldg(v + q + 2 * d.py))
-                         : (DFD_C24_3 * __ldg(v + q - 2 * d.py) - DFD_C24_2 * __ldg(v + q - d.py) + DFD_C24_1 * __ldg(v + q))) *
-                a.rDH;
-      }
-    }
-    float dd[9];
-    dd[0] = dz[0]; dd[1] = dz[1]; dd[2] = dz[2];
-    dd[3] = dv[3]; dd[4] = dv[4]; dd[5] = dv[5]; dd[6] = dv[6]; dd[7] = dv[7]; dd[8] = dv[8];
-    float Dm[9];
-    axis_terms(dd, ez0, ez1, ez2, lam, mu, rrho, Dm);
-#pragma unroll
-    for (int f = 3; f < 9; f++) D[f] = Dm[f];
-  }
+  axis_terms(dv, ez0, ez1, ez2, lam, mu, rrho, D);
 #pragma unroll
   for (int f = 0; f < 9; f++) h[f] += D[f] * rb3;
   if (pz1 || pz2) {
     const int fc = pz1 ? 4 : 5;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
-    pml_face<IRK>(a, fc, qa, st, rb3, __ldg(a.Bz + k), __ldg(a.Dpz + k), __ldg(a.Apz + k), Dz_plain, nullptr,
+    pml_face<IRK>(a, fc, qa, st, rb3, __ldg(a.Bz + k), __ldg(a.Dpz + k), __ldg(a.Apz + k), D, nullptr,
              ez0, ez1, ez2, lam, mu, p);
-  }
-  // ---- traction image for the momentum equation on the top three rows (wave.cu:398-487)
-  if (fs) {
-    int ik = d.nk - 1 - k;
-    float rrhojac = rrho / __ldg(M + 9 * n + q);
-    float v1[3][7], v2[3][7], v3[3][7];
-#pragma unroll
-    for (int l = 0; l < 7; l++) {
-      traction(W, M, n, q + (l - 3) * d.sx, 0, v1[0][l], v1[1][l], v1[2][l]);
-      traction(W, M, n, q + (l - 3), 3, v2[0][l], v2[1][l], v2[2][l]);
-      traction(W, M, n, q + (long long)(l - 3) * d.py, 6, v3[0][l], v3[1][l], v3[2][l]);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      v3[c][ik + 3] = 0.0f;
-      for (int l = 0; l < 3 - ik; l++) v3[c][6 - l] = -v3[c][l + 2 * ik];
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float tx = d5a<FX>(v1[c], 3) * a.rDH, ty = d5a<FY>(v2[c], 3) * a.rDH, tz = d5a<FZ>(v3[c], 3) * a.rDH;
-      h[c] = (tx * rb1 + ty * rb2 + tz * rb3) * rrhojac;
-    }
   }
   // ---- RK4 registers and Cerjan sponge
   float damp = 1.0f;
@@ -186,26 +109,217 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
 }
 
 
-// Shell kernels: the general update on up to eight boxes (PML slabs, free-surface rows)
-// that surround the interior box; one 1-D grid of 128-thread blocks is split over the
-// boxes below the free-surface rows and a second over the rows themselves.  At most 170
-// registers, three blocks per SM: the PML path needs about 160; the traction image of the
-// free-surface rows would take about 230, but the third resident block is worth more than
-// the few values it spills (measured against two and four blocks per SM).  A box at least 32 nodes wide in y and 4 in z is tiled (32 y, 4 z) per block; a
-// thinner box (the y slabs of the PML, the free-surface rows) is flattened over (y, z)
-// with y fastest, so that no thread idles and the y-face PML state (y fastest over N
-// nodes, then z) is read contiguously.
+// The three free-surface rows.  Every node needs jac e . sigma (the traction of an axis) on
+// the five points of each axis's operator: read point by point from memory that is 15 x 10
+// loads a node, and the kernel waited on them (66 us per stage on the 400 x 300 x 200 job).
+// A block takes SJ columns x 3 rows x SI planes, evaluates the tractions once per node of
+// its tile and halo (2.0 to 2.7 evaluations per thread) into shared memory and applies the
+// operators there.
+constexpr int SJ = 16, SI = 4, SURF_THREADS = SJ * 3 * SI;
+struct SurfTile {
+  float t1[3][SI + 4][3][SJ];   // xi traction, halo in x
+  float t2[3][SI][3][SJ + 4];   // eta traction, halo in y
+  float t3[3][SI][6][SJ];       // zeta traction, rows nk - 6 .. nk - 1
+};
+static inline int surface_blocks(const Dims& d) { return ((d.nj + SJ - 1) / SJ) * ((d.ni + SI - 1) / SI); }
+
+template <int FX, int FY, int FZ, int IRK>
+__device__ __forceinline__ void surface_body(const VolArgs& a, int blk, SurfTile& st) {
+  const Dims& d = a.d;
+  constexpr int RX = FX == 1 ? 1 : 3, RY = FY == 1 ? 1 : 3, RZ = FZ == 1 ? 1 : 3;  // centre of each window
+  const int gj = (d.nj + SJ - 1) / SJ;
+  const int tx = threadIdx.x % SJ, zr = threadIdx.x / SJ % 3, xi = threadIdx.x / (3 * SJ);
+  const int jb = (blk % gj) * SJ, ib = (blk / gj) * SI;
+  const int i = ib + xi, j = jb + tx, k = d.nk - 3 + zr;
+  const int i1 = i + 3, j1 = j + 3, k1 = k + 3;
+  const long long n = d.nxyz;
+  const long long q = idx3(d, i1, j1, k1);
+  const float* __restrict__ W = a.Win;
+  const float* __restrict__ M = a.M;
+  float t[3], m[13];
+  // own node (the halo columns and planes of the arrays hold what edge nodes read)
+  if (i1 < d.nx && j1 < d.ny) {
+#pragma unroll
+    for (int e = 0; e < 13; e++) m[e] = __ldg(M + e * n + q);
+    const float txx = __ldg(W + 3 * n + q), tyy = __ldg(W + 4 * n + q), tzz = __ldg(W + 5 * n + q);
+    const float txy = __ldg(W + 6 * n + q), txz = __ldg(W + 7 * n + q), tyz = __ldg(W + 8 * n + q);
+    st.t1[0][xi + RX][zr][tx] = (m[0] * txx + m[1] * txy + m[2] * txz) * m[9];
+    st.t1[1][xi + RX][zr][tx] = (m[0] * txy + m[1] * tyy + m[2] * tyz) * m[9];
+    st.t1[2][xi + RX][zr][tx] = (m[0] * txz + m[1] * tyz + m[2] * tzz) * m[9];
+    st.t2[0][xi][zr][tx + RY] = (m[3] * txx + m[4] * txy + m[5] * txz) * m[9];
+    st.t2[1][xi][zr][tx + RY] = (m[3] * txy + m[4] * tyy + m[5] * tyz) * m[9];
+    st.t2[2][xi][zr][tx + RY] = (m[3] * txz + m[4] * tyz + m[5] * tzz) * m[9];
+    st.t3[0][xi][3 + zr][tx] = (m[6] * txx + m[7] * txy + m[8] * txz) * m[9];
+    st.t3[1][xi][3 + zr][tx] = (m[6] * txy + m[7] * tyy + m[8] * tyz) * m[9];
+    st.t3[2][xi][3 + zr][tx] = (m[6] * txz + m[7] * tyz + m[8] * tzz) * m[9];
+    // z halo: three rows below for the backward operator, one for the forward one
+    if (FZ == -1 || zr == 2) {
+      traction(W, M, n, q - 3LL * d.py, 6, t[0], t[1], t[2]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) st.t3[c][xi][zr][tx] = t[c];
+    }
+  }
+  {
+    // x halo: one of its four planes per thread plane
+    const int px = xi < RX ? xi : xi + SI, ih = ib + px - RX + 3;
+    if (ih < d.nx && j1 < d.ny) {
+      traction(W, M, n, idx3(d, ih, j1, k1), 0, t[0], t[1], t[2]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) st.t1[c][px][zr][tx] = t[c];
+    }
+  }
+  if (tx < 4) {
+    const int col = tx < RY ? tx : tx + SJ, jh = jb + col - RY + 3;
+    if (jh < d.ny && i1 < d.nx) {
+      traction(W, M, n, idx3(d, i1, jh, k1), 3, t[0], t[1], t[2]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) st.t2[c][xi][zr][col] = t[c];
+    }
+  }
+  __syncthreads();
+  if (i >= d.ni || j >= d.nj) return;
+  if (a.united && i1 >= d.i0 - 3 && i1 <= d.i0 + 3 && !a.united[j + k * d.nj]) return;  // band node
+
+  const float lam = m[10], mu = m[11], rrho = 1.0f / m[12];
+  const float rb1 = __ldg(a.rBx + i), rb2 = __ldg(a.rBy + j), rb3 = __ldg(a.rBz + k);
+  const float ez0 = m[6], ez1 = m[7], ez2 = m[8];
+  float h[9], p[9], dv[9], D[9], dxv[3], dyv[3], dz[3];
+#pragma unroll
+  for (int f = 0; f < 9; f++) p[f] = 0.0f;
+  const bool top = k == d.nk - 1;
+  const bool px1 = a.aux[0] && i < d.N, px2 = a.aux[1] && i >= d.ni - d.N;
+  const bool py1 = a.aux[2] && j < d.N, py2 = a.aux[3] && j >= d.nj - d.N;
+  const bool pz1 = a.aux[4] && k < d.N, pz2 = a.aux[5] && k >= d.nk - d.N;
+  // The momentum equation comes from the tractions below, so the stress derivatives are
+  // formed only for the ADE state of a face (D[0..2]).
+#pragma unroll
+  for (int f = 0; f < 9; f++) dv[f] = 0.0f;
+  // ---- x ----
+#pragma unroll
+  for (int f = 0; f < 3; f++) dxv[f] = dv[f] = d5<FX>(W + f * n, q, d.sx) * a.rDH;
+  if (px1 || px2) {
+#pragma unroll
+    for (int f = 3; f < 9; f++) dv[f] = d5<FX>(W + f * n, q, d.sx) * a.rDH;
+  }
+  axis_terms(dv, m[0], m[1], m[2], lam, mu, rrho, D);
+#pragma unroll
+  for (int f = 3; f < 9; f++) h[f] = D[f] * rb1;
+  if (px1 || px2) {
+    if (top) {
+      const float* mx = a.mVx2Vz + (j1 + (long long)i1 * d.ny) * 9;
+#pragma unroll
+      for (int r = 0; r < 3; r++) dz[r] = mx[3 * r] * dxv[0] + mx[3 * r + 1] * dxv[1] + mx[3 * r + 2] * dxv[2];
+    }
+    const int fc = px1 ? 0 : 1;
+    pml_face<IRK>(a, fc, pml_index(d, fc, i, j, k), pml_fstride(d, fc), rb1, __ldg(a.Bx + i), __ldg(a.Dpx + i),
+                  __ldg(a.Apx + i), D, top ? dz : nullptr, ez0, ez1, ez2, lam, mu, p);
+  }
+  // ---- y ----
+#pragma unroll
+  for (int f = 0; f < 3; f++) dyv[f] = dv[f] = d5<FY>(W + f * n, q, 1) * a.rDH;
+  if (py1 || py2) {
+#pragma unroll
+    for (int f = 3; f < 9; f++) dv[f] = d5<FY>(W + f * n, q, 1) * a.rDH;
+  }
+  axis_terms(dv, m[3], m[4], m[5], lam, mu, rrho, D);
+#pragma unroll
+  for (int f = 3; f < 9; f++) h[f] += D[f] * rb2;
+  if (py1 || py2) {
+    if (top) {
+      const float* my = a.mVy2Vz + (j1 + (long long)i1 * d.ny) * 9;
+#pragma unroll
+      for (int r = 0; r < 3; r++) dz[r] = my[3 * r] * dyv[0] + my[3 * r + 1] * dyv[1] + my[3 * r + 2] * dyv[2];
+    }
+    const int fc = py1 ? 2 : 3;
+    pml_face<IRK>(a, fc, pml_index(d, fc, i, j, k), pml_fstride(d, fc), rb2, __ldg(a.By + j), __ldg(a.Dpy + j),
+                  __ldg(a.Apy + j), D, top ? dz : nullptr, ez0, ez1, ez2, lam, mu, p);
+  }
+  // ---- z: a face's ADE state takes the plain derivatives, the stress rates the velocity
+  // derivatives of the top rows (wave.cu:205-245)
+  if (pz1 || pz2) {
+#pragma unroll
+    for (int f = 0; f < 9; f++) dv[f] = d5<FZ>(W + f * n, q, d.py) * a.rDH;
+    axis_terms(dv, ez0, ez1, ez2, lam, mu, rrho, D);
+    const int fc = pz1 ? 4 : 5;
+    pml_face<IRK>(a, fc, pml_index(d, fc, i, j, k), pml_fstride(d, fc), rb3, __ldg(a.Bz + k), __ldg(a.Dpz + k),
+                  __ldg(a.Apz + k), D, nullptr, ez0, ez1, ez2, lam, mu, p);
+  }
+  if (top) {
+    const float* mx = a.mVx2Vz + (j1 + (long long)i1 * d.ny) * 9;
+    const float* my = a.mVy2Vz + (j1 + (long long)i1 * d.ny) * 9;
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+      dv[r] = (mx[3 * r] * dxv[0] + mx[3 * r + 1] * dxv[1] + mx[3 * r + 2] * dxv[2]) +
+              (my[3 * r] * dyv[0] + my[3 * r + 1] * dyv[1] + my[3 * r + 2] * dyv[2]);
+  } else if (k == d.nk - 2) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const float* v = W + r * n;
+      dv[r] = (FZ == 1 ? (__ldg(v + q + d.py) - __ldg(v + q)) : (__ldg(v + q) - __ldg(v + q - d.py))) * a.rDH;
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const float* v = W + r * n;
+      dv[r] = (FZ == 1 ? (-DFD_C24_1 * __ldg(v + q) + DFD_C24_2 * __ldg(v + q + d.py) - DFD_C24_3 * __ldg(v + q + 2 * d.py))
+                       : (DFD_C24_3 * __ldg(v + q - 2 * d.py) - DFD_C24_2 * __ldg(v + q - d.py) + DFD_C24_1 * __ldg(v + q))) *
+              a.rDH;
+    }
+  }
+  axis_terms(dv, ez0, ez1, ez2, lam, mu, rrho, D);
+#pragma unroll
+  for (int f = 3; f < 9; f++) h[f] += D[f] * rb3;
+  // ---- traction image for the momentum equation (wave.cu:398-487): no traction on the top
+  // row, its odd image above
+  const float rrhojac = rrho / m[9];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    float vx[5], vy[5], vz[5];
+#pragma unroll
+    for (int s = 0; s < 5; s++) {
+      vx[s] = st.t1[c][xi + s][zr][tx];
+      vy[s] = st.t2[c][xi][zr][tx + s];
+      const int row = 3 + zr + s - RZ;
+      vz[s] = row == 5 ? 0.0f : row > 5 ? -st.t3[c][xi][10 - row][tx] : st.t3[c][xi][row][tx];
+    }
+    h[c] = (d5w<FX>(vx) * a.rDH * rb1 + d5w<FY>(vy) * a.rDH * rb2 + d5w<FZ>(vz) * a.rDH * rb3) * rrhojac;
+  }
+  // ---- RK4 registers and Cerjan sponge
+  float damp = 1.0f;
+  if (a.dampx) damp = fminf(fminf(__ldg(a.dampx + i1), __ldg(a.dampy + j1)), __ldg(a.dampz + k1));
+  rk_store<IRK>(a, q, h, p, damp);
+}
+template <int FX, int FY, int FZ, int IRK>
+__global__ void __launch_bounds__(SURF_THREADS, 2) volume_surface_kernel(const __grid_constant__ VolArgs a) {
+  __shared__ SurfTile st;
+  surface_body<FX, FY, FZ, IRK>(a, blockIdx.x, st);
+}
+// all scenarios of an ensemble in one launch: scenario s owns blocks [start[s], start[s+1])
+template <int FX, int FY, int FZ, int IRK>
+__global__ void __launch_bounds__(SURF_THREADS, 2)
+    volume_surface_batch(const VolArgs* __restrict__ tab, const int* __restrict__ start, int n) {
+  __shared__ __align__(16) unsigned char raw_a[sizeof(VolArgs)];
+  __shared__ SurfTile st;
+  VolArgs* sa = reinterpret_cast<VolArgs*>(raw_a);
+  int loc;
+  const int sc = scenario_of(start, n, blockIdx.x, &loc);
+  stage_args(sa, tab + sc);
+  __syncthreads();
+  surface_body<FX, FY, FZ, IRK>(*sa, loc, st);
+}
+
+// Shell kernels: the general update on up to six boxes (PML slabs) that surround the plain
+// interior kernel's box; one 1-D grid of 128-thread blocks is split over them.  At most 170
+// registers (the PML path needs about 160), three blocks per SM.  A box at least 32 nodes
+// wide in y and 4 in z is tiled (32 y, 4 z) per block; a thinner box (the y slabs of the
+// PML) is flattened over (y, z) with y fastest, so that no thread idles and the y-face PML
+// state (y fastest over N nodes, then z) is read contiguously.
 constexpr int SHELL_THREADS = 128;
 
-// block blk of the shell grid of one scenario: of the boxes below the free-surface rows
-// (TOP = false, blk counted from box 0) or of the free-surface boxes (TOP, blk counted
-// from box ntop); IRK: the stage (compiled per stage for the free-surface rows), or -1
-template <int FX, int FY, int FZ, bool TOP, int IRK>
+template <int FX, int FY, int FZ>
 __device__ __forceinline__ void volume_shell_body(const VolArgs& a, const Boxes& bx, int blk) {
-  int b = TOP ? bx.ntop : 0;
-  const int bend = TOP ? bx.n : bx.ntop;
-  if (TOP) blk += bx.start[bx.ntop];
-  while (b + 1 < bend && blk >= bx.start[b + 1]) b++;
+  int b = 0;
+  while (b + 1 < bx.ntop && blk >= bx.start[b + 1]) b++;
   int loc = blk - bx.start[b];
   int ni = bx.hi[b][0] - bx.lo[b][0], nj = bx.hi[b][1] - bx.lo[b][1], nk = bx.hi[b][2] - bx.lo[b][2];
   int i, j, k;
@@ -224,15 +338,15 @@ __device__ __forceinline__ void volume_shell_body(const VolArgs& a, const Boxes&
     i = bi;
     if (i >= ni || j >= nj || k >= nk) return;
   }
-  volume_point_general<FX, FY, FZ, TOP, IRK>(a, bx.lo[b][0] + i, bx.lo[b][1] + j, bx.lo[b][2] + k);
+  volume_point_general<FX, FY, FZ, -1>(a, bx.lo[b][0] + i, bx.lo[b][1] + j, bx.lo[b][2] + k);
 }
-template <int FX, int FY, int FZ, bool TOP, int IRK>
+template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(SHELL_THREADS, 3)
     volume_shell_kernel(const __grid_constant__ VolArgs a, const __grid_constant__ Boxes bx) {
-  volume_shell_body<FX, FY, FZ, TOP, IRK>(a, bx, blockIdx.x);
+  volume_shell_body<FX, FY, FZ>(a, bx, blockIdx.x);
 }
 // all scenarios of an ensemble in one launch: scenario s owns blocks [start[s], start[s+1])
-template <int FX, int FY, int FZ, bool TOP, int IRK>
+template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(SHELL_THREADS, 3)
     volume_shell_batch(const VolArgs* __restrict__ tab, const Boxes* __restrict__ boxes,
                        const int* __restrict__ start, int n) {
@@ -245,7 +359,7 @@ __global__ void __launch_bounds__(SHELL_THREADS, 3)
   stage_args(sa, tab + sc);
   stage_args(sb, boxes + sc);
   __syncthreads();
-  volume_shell_body<FX, FY, FZ, TOP, IRK>(*sa, *sb, loc);
+  volume_shell_body<FX, FY, FZ>(*sa, *sb, loc);
 }
 
 // Interior kernel: no PML (beta = 1, no auxiliary state), no free-surface rows.  Each
@@ -414,7 +528,8 @@ VolPlan plan_volume(const VolArgs& a, const TileCtx* tc) {
     bx.start[b] = tot;
     int ni = bx.hi[b][0] - bx.lo[b][0], nj = bx.hi[b][1] - bx.lo[b][1], nk = bx.hi[b][2] - bx.lo[b][2];
     bx.thin[b] = nj < 32 || nk < 4;
-    tot += bx.thin[b] ? ((nj * nk + SHELL_THREADS - 1) / SHELL_THREADS) * ni : ((nj + 31) / 32) * ((nk + 3) / 4) * ni;
+    if (b >= bx.ntop) tot += surface_blocks(d);  // the free-surface rows
+    else tot += bx.thin[b] ? ((nj * nk + SHELL_THREADS - 1) / SHELL_THREADS) * ni : ((nj + 31) / 32) * ((nk + 3) / 4) * ni;
   }
   bx.start[bx.n] = tot;
   pl.shell_blocks = tot;
@@ -444,9 +559,9 @@ static long long launch_flags(const VolArgs& a, cudaStream_t s, cudaStream_t s_s
     cudaStreamWaitEvent(s_shell, *fork, 0);
   }
   const int below = pl.bx.start[pl.bx.ntop], above = pl.bx.start[pl.bx.n] - below;
-  if (below > 0) volume_shell_kernel<FX, FY, FZ, false, -1><<<below, SHELL_THREADS, 0, s_shell>>>(a, pl.bx);
+  if (below > 0) volume_shell_kernel<FX, FY, FZ><<<below, SHELL_THREADS, 0, s_shell>>>(a, pl.bx);
   if (above > 0) {
-#define DFD_L(K) volume_shell_kernel<FX, FY, FZ, true, K><<<above, SHELL_THREADS, 0, s_shell>>>(a, pl.bx)
+#define DFD_L(K) volume_surface_kernel<FX, FY, FZ, K><<<above, SURF_THREADS, 0, s_shell>>>(a)
     DFD_BY_STAGE(a.irk, DFD_L);
 #undef DFD_L
   }
@@ -457,11 +572,11 @@ template <int FX, int FY, int FZ>
 static void shell_batch_t(const VolArgs* tab, const Boxes* boxes, const int* start, int n, int blocks, bool top,
                           int irk, cudaStream_t s) {
   if (top) {
-#define DFD_L(K) volume_shell_batch<FX, FY, FZ, true, K><<<blocks, SHELL_THREADS, 0, s>>>(tab, boxes, start, n)
+#define DFD_L(K) volume_surface_batch<FX, FY, FZ, K><<<blocks, SURF_THREADS, 0, s>>>(tab, start, n)
     DFD_BY_STAGE(irk, DFD_L);
 #undef DFD_L
   } else {
-    volume_shell_batch<FX, FY, FZ, false, -1><<<blocks, SHELL_THREADS, 0, s>>>(tab, boxes, start, n);
+    volume_shell_batch<FX, FY, FZ><<<blocks, SHELL_THREADS, 0, s>>>(tab, boxes, start, n);
   }
 }
 void launch_shell_batch(const VolArgs* tab, const Boxes* boxes, const int* start, int n, int blocks, int FX, int FY,
