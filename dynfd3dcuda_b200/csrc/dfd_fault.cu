@@ -1018,7 +1018,7 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
 }
 
 template <int FY, int FZ>
-__global__ void __launch_bounds__(128) fault_node_kernel(const __grid_constant__ FaultArgs a) {
+__global__ void __launch_bounds__(128, 4) fault_node_kernel(const __grid_constant__ FaultArgs a) {
   __shared__ __align__(16) float snet[4 * NET_PIECES];
   fault_node_body<FY, FZ>(a, blockIdx.x, snet);
 }
@@ -1029,13 +1029,13 @@ __global__ void __launch_bounds__(128) fault_node_kernel(const __grid_constant__
 template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_band_kernel(const __grid_constant__ FaultArgs a) {
   __shared__ BandTile bt;
-  fault_band_body<FX, FY, FZ>(a, blockIdx.x, blockIdx.y, blockIdx.z, bt);
+  fault_band_body<FX, FY, FZ>(a, blockIdx.x, blockIdx.y, 6 - blockIdx.z, bt);
 }
 
 // Batched launches over the scenarios of an ensemble: scenario s owns the blocks
 // [start[s], start[s+1]) of a 1-D grid, laid out as its own (32, 4)-block grid over (NY, NZ).
 template <int FY, int FZ>
-__global__ void __launch_bounds__(128) fault_node_batch(const FaultArgs* __restrict__ tab, const int* __restrict__ start,
+__global__ void __launch_bounds__(128, 4) fault_node_batch(const FaultArgs* __restrict__ tab, const int* __restrict__ start,
                                                         int n) {
   __shared__ __align__(16) float snet[4 * NET_PIECES];
   __shared__ __align__(16) unsigned char raw[sizeof(FaultArgs)];
@@ -1059,7 +1059,7 @@ __global__ void __launch_bounds__(128, 4) fault_band_batch(const FaultArgs* __re
   const FaultArgs& a = *sa;
   const int gx = (a.d.nj + 31) / 32, gxy = gx * ((a.d.nk + 3) / 4);
   // the scenario's blocks: seven parts of its (32, 4)-block grid
-  fault_band_body<FX, FY, FZ>(a, (loc % gxy) % gx, (loc % gxy) / gx, loc / gxy, bt);
+  fault_band_body<FX, FY, FZ>(a, (loc % gxy) % gx, (loc % gxy) / gx, 6 - loc / gxy, bt);
 }
 
 // Thermal pressurisation (thermpress.cu:22-236), once per step before the stages.  Each
