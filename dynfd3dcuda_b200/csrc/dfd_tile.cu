@@ -37,7 +37,7 @@ template <int TR>
 struct TileShape {
   static constexpr int HH = TR + 4, HB = HW * HH, HSLOT = 9 * HB, PB = TJ * TR, QSLOT = 12 * PB;
   static constexpr int PSLOT = 18 * PB;
-  static constexpr int NCW = 2 * TR, NTOT = NCW * 32 + 32;
+  static constexpr int NCW = TR, NTOT = NCW * 32 + 32;
   static constexpr int NS = TR == 8 ? 8 : 6, NP = 3, NQ = 2;  // stencil planes, RK slots, unit planes
   static constexpr int CTAS = TR == 8 ? 1 : 2;
   static constexpr size_t SMEM =
@@ -63,7 +63,7 @@ int tile_ctas_per_sm(int tr) { return tr == 4 ? TileShape<4>::CTAS : TileShape<8
 // scenarios of tab (an ensemble) in one launch; the parameters mp0, a0, sc0 then
 // describe scenario 0 and give the stage's common values.  TR: rows of a tile (TileShape).
 template <int FX, int FY, int FZ, int IRK, bool BATCH, int TR>
-__global__ void __maxnreg__(96)
+__global__ void __maxnreg__(168)
     volume_tile_kernel(const __grid_constant__ TileMaps mp0, const __grid_constant__ VolArgs a0,
                        const __grid_constant__ TileSched sc0, const TileScen* __restrict__ tab, int nscen,
                        int nunits, int* err, int* sched) {
@@ -182,13 +182,14 @@ __global__ void __maxnreg__(96)
     return;
   }
 
-  // ---------------- computing warps: warps w and w + NCW/2 share the row of nodes
-  // (y = lane, z = w): the first computes the momentum equation (velocity fields), the
-  // second the constitutive law (stress fields)
+  // ---------------- computing warps: a warp takes two rows of nodes, a half-warp each, two
+  // neighbouring nodes in y per lane; warps w and w + NCW/2 share the rows: the first
+  // computes the momentum equation (velocity fields), the second the constitutive law
+  // (stress fields)
   const int role = warp >= NCW / 2 ? 1 : 0;
-  const int ty = warp - role * (NCW / 2);
-  const int hc = (ty + RZ) * HW + lane + 4;  // node inside a halo field box
-  const int pc = ty * TJ + lane;             // node inside a pointwise field box
+  const int ty = 2 * (warp - role * (NCW / 2)) + (lane >> 4), tj = 2 * (lane & 15);
+  const int hc = (ty + RZ) * HW + tj + 4;  // first node of the pair inside a halo field box
+  const int pc = ty * TJ + tj;             // the same inside a pointwise field box
   Ring wr, pr, qr;  // next stencil plane to wait for; RK-register slot of the step; unit planes
   int sb = 0;       // slot of the step's first stencil plane
   for (;;) {
@@ -207,15 +208,26 @@ __global__ void __maxnreg__(96)
     const int ntile = sc.ntj * sc.ntk;
     const int tc = lu / ntile, ru = lu % ntile;
     const int ib = sc.lo_x + tc * sc.ci, ie = min(ib + sc.ci, sc.hi_x);
-    const int j = sc.lo_y + (ru % sc.ntj) * TJ + lane, k = sc.lo_z + (ru / sc.ntj) * TK + ty;
-    const bool active = j < sc.hi_y && k < sc.hi_z;
-    const bool band = active && a.united && !a.united[j + k * d.nj];
-    float dyz = 1.0f;
-    if (active && a.dampx) dyz = fminf(__ldg(a.dampy + j + 3), __ldg(a.dampz + k + 3));
+    const int j = sc.lo_y + (ru % sc.ntj) * TJ + tj, k = sc.lo_z + (ru / sc.ntj) * TK + ty;
+    const bool act0 = j < sc.hi_y && k < sc.hi_z, act1 = j + 1 < sc.hi_y && k < sc.hi_z;
+    const bool band0 = act0 && a.united && !a.united[j + k * d.nj];
+    const bool band1 = act1 && a.united && !a.united[j + 1 + k * d.nj];
+    float dyz0 = 1.0f, dyz1 = 1.0f;
+    if (a.dampx) {
+      if (act0) dyz0 = fminf(__ldg(a.dampy + j + 3), __ldg(a.dampz + k + 3));
+      if (act1) dyz1 = fminf(__ldg(a.dampy + j + 4), __ldg(a.dampz + k + 3));
+    }
     const long long qyz = idx3(d, 0, j + 3, k + 3);
     const int nst = ie - ib;
     const float* Q = qs + qr.slot * QSLOT + pc;
-    const float mU = Q[0], mV = Q[PB], ety = Q[2 * PB], etz = Q[3 * PB], zty = Q[4 * PB], ztz = Q[5 * PB];
+    PairMetric g;
+    {
+      const f2 fy = pk(FY * a.rDH), fz = pk(FZ * a.rDH);
+      g.U = lds2(Q); g.V = lds2(Q + PB);
+      g.ey1 = mul2(lds2(Q + 2 * PB), fy); g.ey2 = mul2(lds2(Q + 3 * PB), fy);
+      g.ez1 = mul2(lds2(Q + 4 * PB), fz); g.ez2 = mul2(lds2(Q + 5 * PB), fz);
+    }
+    f2 med0 = 0, med1 = 0;  // momentum: 1/rho; constitutive law: lambda, mu
     // per-plane 1-D factors, loaded one plane ahead so that their latency overlaps a plane
     float rA_next = __ldg(a.rxa + ib + 3);
     float dx_next = a.dampx ? __ldg(a.dampx + ib + 3) : 1.0f;
@@ -237,7 +249,21 @@ __global__ void __maxnreg__(96)
         rA_next = __ldg(a.rxa + i + 4);
         if (a.dampx) dx_next = __ldg(a.dampx + i + 4);
       }
-      if (active && !(band && i + 3 >= d.i0 - 3 && i + 3 <= d.i0 + 3)) {
+      // media of the side of the bimaterial split, re-read where the unit crosses it
+      if (s == 0 || i + 3 == a.nxhalf) {
+        const float* m = Q + (i + 3 < a.nxhalf ? 6 : 9) * PB;
+        if (role == 0) {
+          float r0, r1;
+          upk(lds2(m + 2 * PB), r0, r1);
+          med0 = pk(1.0f / r0, 1.0f / r1);
+        } else {
+          med0 = lds2(m);
+          med1 = lds2(m + PB);
+        }
+      }
+      const bool inband = i + 3 >= d.i0 - 3 && i + 3 <= d.i0 + 3;
+      const bool n0 = act0 && !(band0 && inband), n1 = act1 && !(band1 && inband);
+      if (n0 || n1) {
         const int s1 = sb + 1 == NS ? 0 : sb + 1;
         const int s2 = s1 + 1 == NS ? 0 : s1 + 1;
         const int s3 = s2 + 1 == NS ? 0 : s2 + 1;
@@ -248,21 +274,16 @@ __global__ void __maxnreg__(96)
         const float* xs3 = win + s3 * HSLOT + hc;
         const float* xs4 = win + s4 * HSLOT + hc;
         const float* cur = FX == 1 ? xs1 : xs3;  // plane x itself
-        // metric (xi row from the 1-D factor) and media of the side of the bimaterial split
-        NodeMetric g;
-        g.ex0 = rA; g.ex1 = mU * rA; g.ex2 = mV * rA;
-        g.ey1 = ety; g.ey2 = etz; g.ez1 = zty; g.ez2 = ztz;
-        const int side = i + 3 < a.nxhalf ? 6 : 9;
-        g.lam = Q[side * PB]; g.mu = Q[(side + 1) * PB]; g.rrho = 1.0f / Q[(side + 2) * PB];
-        const float damp = a.dampx ? fminf(dx, dyz) : 1.0f;
+        g.xr = pk(FX * a.rDH * rA);
+        const float dp0 = a.dampx ? fminf(dx, dyz0) : 1.0f, dp1 = a.dampx ? fminf(dx, dyz1) : 1.0f;
         const long long q = qyz + (long long)(i + 3) * d.sx;
-        float hv[9];
+        f2 hv[9];
         if (role == 0) {
-          lean_velocity<FX, FY, FZ, HW, SH::HB>(xs0, xs1, xs2, xs3, xs4, cur, g, a.rDH, hv);
-          rk_tile_store<0, 3, IRK, SH::HB, PB>(a, n, q, cur, P, hv, damp);
+          pair_velocity<FX, FY, FZ, HW, SH::HB>(xs0, xs1, xs2, xs3, xs4, cur, g, med0, hv);
+          rk_pair_store<0, 3, IRK, SH::HB, PB>(a, n, q, cur, P, hv, dp0, dp1, n0, n1);
         } else {
-          lean_stress<FX, FY, FZ, HW, SH::HB>(xs0, xs1, xs2, xs3, xs4, cur, g, a.rDH, hv);
-          rk_tile_store<3, 9, IRK, SH::HB, PB>(a, n, q, cur, P, hv, damp);
+          pair_stress<FX, FY, FZ, HW, SH::HB>(xs0, xs1, xs2, xs3, xs4, cur, g, med0, med1, hv);
+          rk_pair_store<3, 9, IRK, SH::HB, PB>(a, n, q, cur, P, hv, dp0, dp1, n0, n1);
         }
       }
       // release the slots this warp has finished with

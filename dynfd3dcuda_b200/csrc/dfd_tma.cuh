@@ -228,6 +228,170 @@ __device__ __forceinline__ void lean_stress(const float* xs0, const float* xs1, 
 #undef DFD_DERY
 #undef DFD_DERZ
 
+// ---------------- two nodes per thread (packed FP32 pairs, one instruction for both)
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f2 pk(float a) { return pk(a, a); }
+__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 lds2(const float* p) { return *reinterpret_cast<const f2*>(p); }
+
+// F times the one-sided derivative on five points in memory order: with the backward
+// operator's points taken in reverse, both signs use the same five constants, and the sign
+// goes into the metric factor of the axis.
+template <int F>
+__device__ __forceinline__ f2 d5p(f2 v0, f2 v1, f2 v2, f2 v3, f2 v4) {
+  const f2 p0 = F == 1 ? v0 : v4, p1 = F == 1 ? v1 : v3, p3 = F == 1 ? v3 : v1, p4 = F == 1 ? v4 : v0;
+  f2 r = mul2(p0, pk(-DFD_C1));
+  r = fma2(p1, pk(-DFD_C2), r);
+  r = fma2(v2, pk(DFD_C3), r);
+  r = fma2(p3, pk(-DFD_C4), r);
+  return fma2(p4, pk(DFD_C5), r);
+}
+template <int F>
+__device__ __forceinline__ float d5n(float v0, float v1, float v2, float v3, float v4) {
+  const float p0 = F == 1 ? v0 : v4, p1 = F == 1 ? v1 : v3, p3 = F == 1 ? v3 : v1, p4 = F == 1 ? v4 : v0;
+  return fmaf(DFD_C5, p4, fmaf(-DFD_C4, p3, fmaf(DFD_C3, v2, fmaf(-DFD_C2, p1, -DFD_C1 * p0))));
+}
+// along y through the pair at p (its first node at an even column): the points of both nodes
+// come as aligned pairs, each node's operator in scalar (the pairs of an odd shift would
+// have to be put together first)
+template <int F>
+__device__ __forceinline__ f2 d5y(const float* p) {
+  float a, b, c, d, e, f, g, h;
+  if (F == 1) {  // nodes 0, 1 need -1 .. 4
+    upk(lds2(p - 2), a, b);
+    upk(lds2(p), c, d);
+    upk(lds2(p + 2), e, f);
+    g = p[4];
+    return pk(d5n<1>(b, c, d, e, f), d5n<1>(c, d, e, f, g));
+  }
+  // nodes 0, 1 need -3 .. 2
+  a = p[-3];
+  upk(lds2(p - 2), b, c);
+  upk(lds2(p), d, e);
+  upk(lds2(p + 2), f, h);
+  return pk(d5n<-1>(a, b, c, d, e), d5n<-1>(b, c, d, e, f));
+}
+template <int F, int S>
+__device__ __forceinline__ f2 d5z(const float* p) {
+  if (F == 1) return d5p<1>(lds2(p - S), lds2(p), lds2(p + S), lds2(p + 2 * S), lds2(p + 3 * S));
+  return d5p<-1>(lds2(p - 3 * S), lds2(p - 2 * S), lds2(p - S), lds2(p), lds2(p + S));
+}
+
+// Metric of a pair in the interior box: the xi row is xr (1, U, V) with xr = FX / (DH a(x)),
+// the eta and zeta rows (ey, ez) carry FY / DH and FZ / DH.
+struct PairMetric {
+  f2 xr, U, V, ey1, ey2, ez1, ez2;
+};
+#define DFD_PX(f) d5p<FX>(lds2(x0 + (f) * HB), lds2(x1 + (f) * HB), lds2(x2 + (f) * HB), lds2(x3 + (f) * HB), lds2(x4 + (f) * HB))
+#define DFD_PY(f) d5y<FY>(cur + (f) * HB)
+#define DFD_PZ(f) d5z<FZ, PW>(cur + (f) * HB)
+// lean_velocity and lean_stress on a pair; the sums over the metric rows are formed before
+// the media factors (21 products for the six strain rates instead of 36)
+template <int FX, int FY, int FZ, int PW, int HB>
+__device__ __forceinline__ void pair_velocity(const float* x0, const float* x1, const float* x2, const float* x3,
+                                              const float* x4, const float* cur, const PairMetric& g, f2 rrho, f2* hv) {
+  f2 h0, h1, h2, t;
+  h0 = DFD_PX(3);
+  t = DFD_PX(6); h0 = fma2(g.U, t, h0); h1 = t;
+  t = DFD_PX(7); h0 = fma2(g.V, t, h0); h2 = t;
+  t = DFD_PX(4); h1 = fma2(g.U, t, h1);
+  t = DFD_PX(8); h1 = fma2(g.V, t, h1); h2 = fma2(g.U, t, h2);
+  t = DFD_PX(5); h2 = fma2(g.V, t, h2);
+  h0 = mul2(h0, g.xr); h1 = mul2(h1, g.xr); h2 = mul2(h2, g.xr);
+  t = DFD_PY(4); h1 = fma2(g.ey1, t, h1);
+  t = DFD_PY(5); h2 = fma2(g.ey2, t, h2);
+  t = DFD_PY(6); h0 = fma2(g.ey1, t, h0);
+  t = DFD_PY(7); h0 = fma2(g.ey2, t, h0);
+  t = DFD_PY(8); h1 = fma2(g.ey2, t, h1); h2 = fma2(g.ey1, t, h2);
+  t = DFD_PZ(4); h1 = fma2(g.ez1, t, h1);
+  t = DFD_PZ(5); h2 = fma2(g.ez2, t, h2);
+  t = DFD_PZ(6); h0 = fma2(g.ez1, t, h0);
+  t = DFD_PZ(7); h0 = fma2(g.ez2, t, h0);
+  t = DFD_PZ(8); h1 = fma2(g.ez2, t, h1); h2 = fma2(g.ez1, t, h2);
+  hv[0] = mul2(h0, rrho); hv[1] = mul2(h1, rrho); hv[2] = mul2(h2, rrho);
+}
+template <int FX, int FY, int FZ, int PW, int HB>
+__device__ __forceinline__ void pair_stress(const float* x0, const float* x1, const float* x2, const float* x3,
+                                            const float* x4, const float* cur, const PairMetric& g, f2 lam, f2 mu,
+                                            f2* hv) {
+  f2 d0, d1, d2, s01, s02, s12, t;
+  t = DFD_PX(0); d0 = t; s01 = mul2(g.U, t); s02 = mul2(g.V, t);
+  t = DFD_PX(1); d1 = mul2(g.U, t); s01 = add2(s01, t); s12 = mul2(g.V, t);
+  t = DFD_PX(2); d2 = mul2(g.V, t); s02 = add2(s02, t); s12 = fma2(g.U, t, s12);
+  d0 = mul2(d0, g.xr); d1 = mul2(d1, g.xr); d2 = mul2(d2, g.xr);
+  s01 = mul2(s01, g.xr); s02 = mul2(s02, g.xr); s12 = mul2(s12, g.xr);
+  t = DFD_PY(0); s01 = fma2(g.ey1, t, s01); s02 = fma2(g.ey2, t, s02);
+  t = DFD_PY(1); d1 = fma2(g.ey1, t, d1); s12 = fma2(g.ey2, t, s12);
+  t = DFD_PY(2); d2 = fma2(g.ey2, t, d2); s12 = fma2(g.ey1, t, s12);
+  t = DFD_PZ(0); s01 = fma2(g.ez1, t, s01); s02 = fma2(g.ez2, t, s02);
+  t = DFD_PZ(1); d1 = fma2(g.ez1, t, d1); s12 = fma2(g.ez2, t, s12);
+  t = DFD_PZ(2); d2 = fma2(g.ez2, t, d2); s12 = fma2(g.ez1, t, s12);
+  const f2 m2 = add2(mu, mu), tr = mul2(lam, add2(add2(d0, d1), d2));
+  hv[3] = fma2(m2, d0, tr); hv[4] = fma2(m2, d1, tr); hv[5] = fma2(m2, d2, tr);
+  hv[6] = mul2(mu, s01); hv[7] = mul2(mu, s02); hv[8] = mul2(mu, s12);
+}
+#undef DFD_PX
+#undef DFD_PY
+#undef DFD_PZ
+
+// rk_tile_store on a pair; n0, n1: which of the two nodes are updated
+template <int F0, int F1, int IRK, int HB, int PBB>
+__device__ __forceinline__ void rk_pair_store(const VolArgs& a, long long n, long long q, const float* cur,
+                                              const float* P, const f2* hv, float damp0, float damp1, bool n0, bool n1) {
+  const f2 damp = pk(damp0, damp1), rka = pk(a.rka), rkb = pk(a.rkb);
+  f2 rd;
+  if (IRK == 2) rd = pk(rk_rd(damp0), rk_rd(damp1));
+  auto put = [&](float* x, f2 v) {
+    if (n0 && n1) {
+      *reinterpret_cast<f2*>(x) = v;
+    } else {
+      float v0, v1;
+      upk(v, v0, v1);
+      if (n0) x[0] = v0;
+      if (n1) x[1] = v1;
+    }
+  };
+#pragma unroll
+  for (int f = F0; f < F1; f++) {
+    const long long x = f * n + q;
+    f2 w;
+    if (IRK == 0) {
+      w = fma2(rka, hv[f], lds2(cur + f * HB));
+    } else if (IRK == 1) {
+      w = fma2(rka, hv[f], lds2(P + f * PBB));
+    } else if (IRK == 2) {
+      const f2 y0 = lds2(P + f * PBB), ny0 = mul2(y0, pk(-1.0f));
+      const f2 u = fma2(lds2(P + (9 + f) * PBB), rd, ny0), v = fma2(lds2(cur + f * HB), rd, ny0);
+      const f2 s = fma2(pk(2.0f), v, u);
+      put(a.T + x, fma2(rkb, hv[f], fma2(s, pk(1.0f / 3.0f), y0)));
+      w = fma2(rka, hv[f], y0);
+    } else {
+      w = fma2(rkb, hv[f], lds2(P + f * PBB));
+    }
+    put(a.Wout + x, mul2(w, damp));
+  }
+}
+
 // first scenario of a batched launch whose units include the global unit u
 __device__ __forceinline__ int tile_scenario(const TileScen* tab, int n, int u) {
   int lo = 0, hi = n;  // tab[lo].unit0 <= u < tab[hi].unit0
