@@ -181,7 +181,10 @@ __device__ double newton_rs(double x, double psi, double ra, double Vhat, double
   return xn;
 }
 
-// Body of the fault node kernel for the block (bx, by) of a (32, 4) grid over (NY, NZ);
+// Body of the fault node kernel for block blk of 128 nodes of the rectangle.  Bound: memory
+// latency (a few hundred bytes a node, one wave of blocks); with every load ahead of the first
+// store a stage takes 15 us on 200 x 100 fault nodes (25.5 with the stores in between) and
+// 18 us on 400 x 200 (27).
 // snet is the block's shared copy of the learned-guess weights.
 template <int FY, int FZ>
 __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, float* snet) {
@@ -663,7 +666,10 @@ __device__ __forceinline__ void rk_store9(const FaultArgs& a, long long q, const
 }
 
 // Traction planes of a block's 32 x 4 nodes of one off-fault layer, with the halo of the y
-// (T2 = jac eta . sigma) and z (T3 = jac zeta . sigma) operators.
+// (T2 = jac eta . sigma) and z (T3 = jac zeta . sigma) operators.  The kernel waits on memory:
+// evaluated point by point the tractions are 210 loads a node and layer, from the tile about
+// 30 (36 -> 25 us per stage on 200 x 100 fault nodes, 88 -> 67 on 400 x 200, with the split
+// nodes, the longest part, at the front of the grid).
 struct BandTile {
   float t2[3][4][36], t3[3][8][32];
 };
@@ -1017,6 +1023,9 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
   fault_to_volume(a, wv, t1c, mq, a.Wout, j1, k1, damp0);
 }
 
+// Four blocks per SM: at the 164 to 180 registers the compiler would take, two or three are
+// resident and a fault of 400 x 200 nodes leaves a nearly empty second wave (27 us; 18 us with
+// the 70 to 160 bytes spilled at 128 registers).
 template <int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_node_kernel(const __grid_constant__ FaultArgs a) {
   __shared__ __align__(16) float snet[4 * NET_PIECES];
@@ -1074,7 +1083,8 @@ __global__ void __launch_bounds__(128, 4) fault_band_batch(const FaultArgs* __re
 // two (NZ, NY) planes, which the friction law and the outputs read.
 
 // per-node scalars of the scheme (thermpress.cu:150-175), as the reference rounds them; the
-// sub-steps multiply by the FP64 reciprocals rdh2 and rfden, formed once per node
+// sub-steps multiply by the FP64 reciprocals rdh2 and rfden, formed once per node (two FP64
+// divisions a point and sub-step were most of the kernel: 55 -> 24 us with 64-point columns)
 struct TpNode {
   float rate, Tau_n, fr, ahy, dh, dh2, dt;
   int nsub;

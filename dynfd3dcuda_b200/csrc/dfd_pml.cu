@@ -9,8 +9,16 @@
 // plane, the stencil input with its halo, the RK registers and the ADE state of one PML
 // face (its "own" face: x for the x slabs, y for the strips, z for the z tiles); a node
 // that also lies in another face (edges and corners of the slabs) reads that face's
-// state from global memory.  One computing warp per row of nodes
-// integrates all nine fields and their PML state.
+// state from global memory.  Two computing warps per row of nodes: one
+// integrates the velocities, the other the stresses, each with its PML state.
+//
+// Bound: latency and issue slots (0.55 to 0.59 instructions issued per cycle and scheduler, a
+// third of the stall cycles on global loads, DRAM at 20 to 31 % of its rate).  One warp per row
+// left two warps on a scheduler: against it, with the same units, a whole run of the 200 x
+// 100 x 100 job takes 35.7 instead of 36.4 ms and of eight mixed scenarios 175.9 instead of
+// 185.0.  Two nodes per lane in packed arithmetic, as the interior kernel has them, halve the
+// instructions and again leave two warps on a scheduler: 34.8 ms on the same job where this
+// form, with the same other kernels, takes 30.4.
 //
 // Right-hand side with the ADE CFS-PML as in the reference's wave.cu:8-204 and
 // pmlx.cu:8-214 / pmly.cu / pmlz.cu, the RK4 registers as rk4.cu:20-33 and 154-257.
@@ -289,10 +297,10 @@ __device__ __forceinline__ void pml_node(const VolArgs& a, int PW, const float* 
   rk_tile_store<H0, H1, IRK>(a, a.d.nxyz, q, cur, P, hv, damp);
 }
 
-// Warp PCW issues the copies; warps 0..PCW-1 compute, one per row of nodes, all nine
-// fields (the lean interior path for a warp whose nodes lie in no PML slab).  The nine warps
-// allow 168 registers a thread (three warps on one of the SM's four 16 K-register
-// partitions), what the ADE path needs without spilling.  Rings as in the interior
+// Warp PCW issues the copies; warps 0..PCW-1 compute, two per row of nodes (the lean interior
+// path for a warp whose nodes lie in no PML slab).  The 17 warps allow 96 registers a thread
+// (five warps on one of the SM's four 16 K-register partitions); with the role and the stage
+// known at compile time the ADE path spills at most 12 bytes.  Rings as in the interior
 // kernel, with shallower rings (PmlRing): a pointwise slot also holds the own face's ADE
 // state.
 // IRK: the RK stage, compiled per stage as in the interior kernel.  BATCH: the units of

@@ -8,12 +8,19 @@
 //   - the pointwise streams of the node: 12 metric/media fields, and the RK registers
 //     W0 (stages 1, 2), the stage-1 input (stage 2) and T (stage 3): TMA boxes (32, 8, 1, n)
 //     in a ring of NP slots.
-// A dedicated warp issues the copies ahead of the sixteen (eight) computing warps (full/empty
+// A dedicated warp issues the copies ahead of the eight (four) computing warps (full/empty
 // mbarrier pairs per slot, no block-wide barrier in the loop), so HBM traffic stays in
 // flight while the stencils are evaluated from shared memory with immediate offsets.
 // No node of the box lies in a PML slab or the free-surface rows (dfd_pml.cu and the
 // general kernel take those).  Outputs (Wout, and T at stage 2) are written straight from
 // registers.
+//
+// Bound: issue slots first (67-69 % of the cycles issued with one node per lane, DRAM at
+// 55-60 %), so a lane updates two neighbouring nodes with packed FP32 instructions and 64-bit
+// accesses: half the instructions and half the warps for the same tile.  With 24 M nodes
+// (400 x 300 x 200) a stage went from 537 / 604 / 708 / 606 us to 458 / 525 / 692 / 524 us,
+// with 2 M nodes (200 x 100 x 100) from 43 / 48 / 57 / 47 to 38 / 43 / 55 / 44 us.  What is
+// left at full size is memory: 117 bytes a node and stage and the stencil halo.
 //
 // The kernel is persistent: one CTA per SM (two with 4-row tiles) takes units (tile column x chunk) from a global
 // counter, and its copy stream runs across unit boundaries, so the next unit's planes
@@ -29,8 +36,8 @@
 namespace dfd {
 
 namespace {
-// Shape of the interior kernel's tiles: 32 (y) x TR (z) nodes.  TR = 8: 16 computing warps
-// and one CTA per SM; TR = 4: 8 computing warps, shallower stencil ring and two CTAs per
+// Shape of the interior kernel's tiles: 32 (y) x TR (z) nodes.  TR = 8: 8 computing warps
+// and one CTA per SM; TR = 4: 4 computing warps, shallower stencil ring and two CTAs per
 // SM (each within half of the SM's 228 KB of shared memory, 1 KB of it reserved per CTA).
 // An RK slot holds W0 and the stage-1 input (stage 2), W0 (stage 1) or T alone (stage 3).
 template <int TR>
@@ -50,13 +57,13 @@ struct TileShape {
 
 int tile_ctas_per_sm(int tr) { return tr == 4 ? TileShape<4>::CTAS : TileShape<8>::CTAS; }
 
-// Warp NCW issues the copies; warps 0..NCW-1 compute one node each per plane (NCW = 2 TR).  Each ring
+// Warp NCW issues the copies; warps 0..NCW-1 compute two nodes per lane and plane (NCW = TR).  Each ring
 // slot has a "full" barrier (completed by the copy's transaction bytes) and an "empty"
 // barrier (one arrival per computing warp once it has finished reading the slot).  Three
 // rings: stencil planes (NS), RK registers of the step (NP; none at stage 0, whose
 // step-start values are the stencil input), metric/media planes of the unit (NQ).  At
-// most 96 registers: with 8-row tiles the 17 warps are spread over the SM's four 16 K-register
-// partitions, five warps on one of them; with 4-row tiles two CTAs of 9 warps share them.
+// most 168 registers (the pairs take 106 to 132): with 8-row tiles the 9 warps put three on one
+// of the SM's four 16 K-register partitions; with 4-row tiles two CTAs of 5 warps share them.
 
 // IRK: the RK stage (a0.irk), a compile-time constant so that each stage's code and
 // register allocation carry only its own RK registers.  BATCH: the units of the nscen

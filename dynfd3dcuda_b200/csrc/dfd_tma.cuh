@@ -14,15 +14,13 @@
 namespace dfd {
 
 namespace {
-constexpr int TJ = TILE_J, TK = TILE_K, NTHR = TJ * TK;
+constexpr int TJ = TILE_J, TK = TILE_K;
 constexpr int HW = TJ + 8;           // halo box width (y): 4 nodes each side (16-byte aligned)
 constexpr int HH = TK + 4;           // halo box height (z): 1 + 3 rows, side set by the z operator
 constexpr int HBOX = HW * HH;        // floats per field of a halo box
 constexpr int HSLOT = 9 * HBOX;      // floats per stencil plane slot
 constexpr int PB = TJ * TK;          // floats per field of a pointwise box
 constexpr int QSLOT = 12 * PB;       // metric / media planes of a unit: U V ety etz zty ztz, 2 x (lam mu rho)
-constexpr int NCW = 2 * NTHR / 32;   // computing warps: two per 32-node row of the tile
-constexpr int NTOT = NCW * 32 + 32;  // plus one copy-issuing warp
 constexpr long long WAIT_LIMIT = 1LL << 22;  // polls of one mbarrier before giving up
 constexpr long long DRILL_LIMIT = 1LL << 12; // the same in the test drill of the bounded waits
 static_assert((HSLOT * 4) % 128 == 0 && (QSLOT * 4) % 128 == 0 && (PB * 4) % 128 == 0, "slot alignment");
