@@ -291,9 +291,9 @@ struct alignas(64) TileScen {
   TileMaps mp;
   TileUnit u;
 };
-// Boxes of the general (shell) kernels: up to eight, each flattened or tiled.  Boxes
-// [0, ntop) lie below the free-surface rows (PML slabs, alignment columns) and go to the
-// kernel without the free-surface terms; boxes [ntop, n) hold the free-surface rows.
+// Boxes of the general (shell) kernel, each flattened or tiled: boxes [0, ntop) lie below the
+// free-surface rows (PML slabs).  Box ntop, where there is one, holds the free-surface rows,
+// which go to a kernel of their own (start counts its blocks).
 struct Boxes {
   int n, ntop;
   int lo[8][3], hi[8][3];  // (i, j, k) interior-index bounds, half open
