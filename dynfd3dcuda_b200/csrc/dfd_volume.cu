@@ -45,7 +45,7 @@ __device__ __forceinline__ void traction(const float* __restrict__ W, const floa
 
 // General node update below the free-surface rows: PML faces and sponge.  Used for the
 // shell of the domain outside the plain interior kernel's box.
-template <int FX, int FY, int FZ, int IRK>
+template <int FX, int FY, int FZ>
 __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, int j, int k) {
   const Dims& d = a.d;
   int i1 = i + 3, j1 = j + 3, k1 = k + 3;
@@ -75,7 +75,7 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
   if (px1 || px2) {
     const int fc = px1 ? 0 : 1;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
-    pml_face<IRK>(a, fc, qa, st, rb1, __ldg(a.Bx + i), __ldg(a.Dpx + i), __ldg(a.Apx + i), D,
+    pml_face<-1>(a, fc, qa, st, rb1, __ldg(a.Bx + i), __ldg(a.Dpx + i), __ldg(a.Apx + i), D,
              nullptr, ez0, ez1, ez2, lam, mu, p);
   }
   // ---- y ----
@@ -87,7 +87,7 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
   if (py1 || py2) {
     const int fc = py1 ? 2 : 3;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
-    pml_face<IRK>(a, fc, qa, st, rb2, __ldg(a.By + j), __ldg(a.Dpy + j), __ldg(a.Apy + j), D,
+    pml_face<-1>(a, fc, qa, st, rb2, __ldg(a.By + j), __ldg(a.Dpy + j), __ldg(a.Apy + j), D,
              nullptr, ez0, ez1, ez2, lam, mu, p);
   }
   // ---- z ----
@@ -99,13 +99,13 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
   if (pz1 || pz2) {
     const int fc = pz1 ? 4 : 5;
     const long long st = pml_fstride(d, fc), qa = pml_index(d, fc, i, j, k);
-    pml_face<IRK>(a, fc, qa, st, rb3, __ldg(a.Bz + k), __ldg(a.Dpz + k), __ldg(a.Apz + k), D, nullptr,
+    pml_face<-1>(a, fc, qa, st, rb3, __ldg(a.Bz + k), __ldg(a.Dpz + k), __ldg(a.Apz + k), D, nullptr,
              ez0, ez1, ez2, lam, mu, p);
   }
   // ---- RK4 registers and Cerjan sponge
   float damp = 1.0f;
   if (a.dampx) damp = fminf(fminf(__ldg(a.dampx + i1), __ldg(a.dampy + j1)), __ldg(a.dampz + k1));
-  rk_store<IRK>(a, q, h, p, damp);
+  rk_store<-1>(a, q, h, p, damp);
 }
 
 
@@ -339,7 +339,7 @@ __device__ __forceinline__ void volume_shell_body(const VolArgs& a, const Boxes&
     i = bi;
     if (i >= ni || j >= nj || k >= nk) return;
   }
-  volume_point_general<FX, FY, FZ, -1>(a, bx.lo[b][0] + i, bx.lo[b][1] + j, bx.lo[b][2] + k);
+  volume_point_general<FX, FY, FZ>(a, bx.lo[b][0] + i, bx.lo[b][1] + j, bx.lo[b][2] + k);
 }
 template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(SHELL_THREADS, 3)
