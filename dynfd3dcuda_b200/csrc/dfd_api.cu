@@ -357,9 +357,9 @@ int dfd_create(const dfd_params* p, int device, dfd_ctx** out) {
   if (!rc) rc = dalloc(ctx, &ctx->tile_err, 1);
   if (!rc) rc = dalloc(ctx, &ctx->tile_sched, 4);  // unit and finished-CTA counters: interior, PML
   if (rc) { dfd_destroy(ctx); return rc; }
-  // volume kernels: DFD_TILE=0 plain interior kernel + general kernel on the PML slabs
-  // and free-surface rows; otherwise (default) the TMA-staged interior and PML kernels
-  // + the general kernel on the free-surface rows
+  // volume kernels: DFD_TILE=0 plain interior kernel + general kernel on the PML slabs;
+  // otherwise (default) the TMA-staged interior and PML kernels; the free-surface kernel
+  // on its rows with both
   const char* tv = getenv("DFD_TILE");
   const int mode = tv && tv[0] == '0' ? 0 : 1;
   float* auxb[6];
@@ -763,7 +763,8 @@ static int enqueue_stage(dfd_ctx* ctx, int pattern, int irk, cudaEvent_t* vb = n
   }
   if (vb) cudaEventRecord(*vb, ctx->s0);
   if (ctx->serial) {
-    // interior and PML kernels on s0; then the general kernel (free-surface rows) on s2
+    // interior and PML kernels on s0; then the free-surface kernel (plain path: the general one
+    // on the slabs too) on s2
     // beside the fault band kernel on s0: two small latency-bound kernels that fit on the
     // SMs together
     VolArgs va = vol_args(ctx, pattern, irk);
@@ -1601,9 +1602,9 @@ int dfd_output_close(dfd_ctx* ctx) {
 
 // ------------------------------------------------------------------ ensemble --
 // A batch of prepared scenarios (contexts on one device) stepped together: per RK stage
-// one batched launch each of the fault node, fault band and general (shell) kernels over
-// every scenario, and one persistent launch of the tiled interior kernel whose units span
-// all scenarios.  The per-stage argument tables live in device memory (one set per flag
+// one batched launch each of the fault node, fault band and free-surface kernels over every
+// scenario (and of the general kernel, on the plain path), and one persistent launch each of
+// the tiled interior and PML kernels whose units span all scenarios.  The per-stage argument tables live in device memory (one set per flag
 // pattern and stage); each step is replayed from a CUDA graph.  Scenario state stays in
 // the scenarios' own contexts, so results are read with the usual getters.
 struct EnsStage {
@@ -1614,9 +1615,9 @@ struct EnsStage {
   int bblocks = 0;
   VolArgs* vol = nullptr;      // all scenarios
   Boxes* boxes = nullptr;
-  int* sstart = nullptr;       // (n + 1) block starts of the shell kernel, boxes below the top rows
+  int* sstart = nullptr;       // (n + 1) block starts of the general kernel (plain path)
   int sblocks = 0;
-  int* tstart = nullptr;       // (n + 1) block starts of the shell kernel, free-surface rows
+  int* tstart = nullptr;       // (n + 1) block starts of the free-surface kernel
   int tblocks = 0;
   TileScen* tile = nullptr;    // all scenarios, interior kernel
   TileScen first;              // scenario 0, passed by value (stage-wide values)
@@ -1771,7 +1772,7 @@ static int ens_enqueue(dfd_ens* e, int pat, int irk) {
     launch_tile_batch(S.first, S.tile, n, S.nunits, e->nsm, e->tr, S.FX, S.FY, S.FZ, e->err, e->sched, e->s0);
     launch_pml_batch(S.pfirst, S.ptile, n, S.punits, e->nsm, S.FX, S.FY, S.FZ, e->err, e->sched, S.nunits > 0,
                      e->s0);
-    // the general kernel beside the fault band kernel
+    // the free-surface kernel (plain path: the general one too) beside the fault band kernel
     cudaEventRecord(e->ev_fork, e->s0);
     cudaStreamWaitEvent(e->s2, e->ev_fork, 0);
     launch_shell_batch(S.vol, S.boxes, S.sstart, n, S.sblocks, S.FX, S.FY, S.FZ, false, irk, e->s2);

@@ -182,9 +182,11 @@ __device__ double newton_rs(double x, double psi, double ra, double Vhat, double
 }
 
 // Body of the fault node kernel for block blk of 128 nodes of the rectangle.  Bound: memory
-// latency (a few hundred bytes a node, one wave of blocks); with every load ahead of the first
-// store a stage takes 15 us on 200 x 100 fault nodes (25.5 with the stores in between) and
-// 18 us on 400 x 200 (27).
+// latency (a few hundred bytes a node, 0.15 to 0.18 instructions issued per cycle and
+// scheduler).  With every load ahead of the first store a stage went from 25.5 to 14.5 us on
+// 200 x 100 fault nodes (77 blocks) and, at the registers that the compiler then took, stayed
+// at 25 to 29 us on 400 x 200 (27 before): those blocks no longer fit in one wave, see the
+// bound at the kernel.
 // snet is the block's shared copy of the learned-guess weights.
 template <int FY, int FZ>
 __device__ __forceinline__ void fault_node_body(const FaultArgs& a, int blk, float* snet) {
@@ -1024,8 +1026,10 @@ __device__ __forceinline__ void fault_band_body(const FaultArgs& a, int bx, int 
 }
 
 // Four blocks per SM: at the 164 to 180 registers the compiler would take, two or three are
-// resident and a fault of 400 x 200 nodes leaves a nearly empty second wave (27 us; 18 us with
-// the 70 to 160 bytes spilled at 128 registers).
+// resident and the 451 blocks of a fault of 400 x 200 nodes leave a nearly empty second wave (25
+// to 29 us; 18 us with the 70 to 160 bytes spilled at 128 registers, where 592 blocks are
+// resident).  A small fault, one wave either way, pays for the spills: 14.5 -> 15.4 us on 200 x
+// 100.  A larger one takes several waves (1000 x 300: 1981 blocks, 60 us).
 template <int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_node_kernel(const __grid_constant__ FaultArgs a) {
   __shared__ __align__(16) float snet[4 * NET_PIECES];
@@ -1033,8 +1037,8 @@ __global__ void __launch_bounds__(128, 4) fault_node_kernel(const __grid_constan
 }
 // grid z: the part (six off-fault layers, then the split nodes), so that the seven
 // independent pieces of a fault column run in parallel.  At most 128 registers (four
-// blocks per SM): this latency-bound kernel gains more from the resident warps than it
-// loses to the few spilled values (measured: 3, 4, 5, 6 blocks per SM).
+// blocks per SM): this latency-bound kernel gains more from the resident warps than its
+// batched form loses to the 28 to 48 bytes it spills (measured: 3, 4, 5, 6 blocks per SM).
 template <int FX, int FY, int FZ>
 __global__ void __launch_bounds__(128, 4) fault_band_kernel(const __grid_constant__ FaultArgs a) {
   __shared__ BandTile bt;

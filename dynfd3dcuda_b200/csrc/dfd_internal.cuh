@@ -301,7 +301,7 @@ struct Boxes {
   int start[9];            // first block of each box
 };
 // Volume work of one stage of one scenario: the box of the tiled (or plain) interior
-// kernel, the units of the tiled PML kernel and the general kernel's boxes.
+// kernel, the units of the tiled PML kernel and the boxes of the other two.
 struct VolPlan {
   bool tiled, plain;
   int3 lo, hi;        // interior-kernel box
@@ -329,7 +329,8 @@ void launch_pml_batch(const TileScen& first, const TileScen* tab, int n, int nun
 // batched launches (dfd_volume.cu, dfd_tile.cu, dfd_fault.cu)
 void launch_tile_batch(const TileScen& first, const TileScen* tab, int n, int nunits, int grid, int tr, int FX,
                        int FY, int FZ, int* err, int* sched, cudaStream_t s);
-// top: the free-surface boxes (start: per-scenario block starts of those), else the others;
+// top: the free-surface kernel (start: per-scenario block starts of its rows), else the
+// general kernel on the slabs of the plain path;
 // irk: the stage of every scenario's arguments
 void launch_shell_batch(const VolArgs* tab, const Boxes* boxes, const int* start, int n, int blocks, int FX, int FY,
                         int FZ, bool top, int irk, cudaStream_t s);

@@ -1,6 +1,6 @@
 // Nodes of the volume stage below the free-surface rows that the interior kernel does
 // not take, staged through shared memory by TMA: the PML slabs of all six faces and the
-// nodes that fill their tiles (the interior kernel takes whole tiles only).
+// nodes between them and the interior kernel's box.
 //
 // Units (dfd_internal.cuh, TileSched): every 32 x 8 tile of the two x slabs, one unit
 // per tile and slab; then, in chunks of x planes between the slabs, the 16 x 16 strip
@@ -12,8 +12,9 @@
 // state from global memory.  Two computing warps per row of nodes: one
 // integrates the velocities, the other the stresses, each with its PML state.
 //
-// Bound: latency and issue slots (0.55 to 0.59 instructions issued per cycle and scheduler, a
-// third of the stall cycles on global loads, DRAM at 20 to 31 % of its rate).  One warp per row
+// Bound: latency and issue slots: 0.62 / 0.57 / 0.47 / 0.55 instructions issued per cycle and
+// scheduler at stages 0 to 3 (320 x 160 x 160 nodes, PML 20), the largest stall on global loads
+// (1.8 to 3.7 cycles an instruction), DRAM at 33 / 47 / 56 / 45 % of its peak.  One warp per row
 // left two warps on a scheduler: against it, with the same units, a whole run of the 200 x
 // 100 x 100 job takes 35.7 instead of 36.4 ms and of eight mixed scenarios 175.9 instead of
 // 185.0.  Two nodes per lane in packed arithmetic, as the interior kernel has them, halve the
@@ -231,10 +232,6 @@ __device__ __forceinline__ void role_terms(const float* dv, float e0, float e1, 
   }
 }
 
-// One node, all nine fields: the three axes with their 1/beta, the ADE state of the faces
-// the node lies in (fx, fy, fz; -1: none; own: the staged face, read from A), the RK4
-// store.  PW: row pitch of the stencil box (40 for 32 x 8 tiles, 24 for strips).  g: separable metric (xi = (1, U, V)/a(x), eta = (0, ety, etz), zeta = (0, zty,
-// ztz)) and media.
 // one-sided 5-point operator along a shared-memory line with a runtime stride
 template <int F>
 __device__ __forceinline__ float d5r(const float* p, int S) {
@@ -272,6 +269,10 @@ __device__ __forceinline__ void pml_axis(const VolArgs& a, const float* dv, floa
     if (face >= 0) role_face<6, AX, IRK>(a, face, face == own, A, i, j, k, rb, dd, al, D, hv + 3);
   }
 }
+// One node, the fields of one role: the three axes with their 1/beta, the ADE state of the
+// faces the node lies in (fx, fy, fz; -1: none; own: the staged face, read from A), the RK4
+// store.  PW: row pitch of the stencil box (40 for 32 x 8 tiles, 24 for strips).  g: separable
+// metric (xi = (1, U, V)/a(x), eta = (0, ety, etz), zeta = (0, zty, ztz)) and media.
 template <int ROLE, int FX, int FY, int FZ, int IRK>
 __device__ __forceinline__ void pml_node(const VolArgs& a, int PW, const float* x0, const float* x1, const float* x2,
                                          const float* x3, const float* x4, const float* cur, const NodeMetric& g,

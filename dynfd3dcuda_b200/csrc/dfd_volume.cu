@@ -5,7 +5,7 @@
 // the classic RK4 register update (rk4.cu:20-33,154-257) and the Cerjan sponge
 // (cerjan.cu:166-200).  The right-hand side never reaches HBM: each stage reads the
 // stencil input (9 fields), the 12 metric/media fields and its RK registers, and writes
-// its output and accumulator -- 39/57/57/39 floats per node for stages 0..3.
+// its output and, at stage 2, the accumulator -- 30/39/57/39 floats per node for stages 0..3.
 //
 // Nodes of the seven x-layers around the fault whose (j,k) is not "united" are left
 // to the band kernel (dfd_fault.cu), exactly the nodes whose right-hand side the
@@ -112,10 +112,12 @@ __device__ __forceinline__ void volume_point_general(const VolArgs& a, int i, in
 // The three free-surface rows.  Every node needs jac e . sigma (the traction of an axis) on
 // the five points of each axis's operator: read point by point from memory that is 15 x 10
 // loads a node, and the kernel waited on them (66 us per stage on the 400 x 300 x 200 job,
-// 20.5 on 200 x 100 x 100; 45 and 16 now, still latency: 12 warps per SM, DRAM at 18 %).
+// 20.5 on 200 x 100 x 100; 47 and 17 now, still latency: 12 warps per SM, 0.3 instructions
+// issued per cycle and scheduler, DRAM at 14 to 19 % of its peak).
 // A block takes SJ columns x 3 rows x SI planes, evaluates the tractions once per node of
-// its tile and halo (2.0 to 2.7 evaluations per thread) into shared memory and applies the
-// operators there.
+// its tile and halo into shared memory (per thread its own node, a node of the x halo, a
+// quarter of one of the y halo and a third (forward z operator) or all of one of the z halo:
+// 2.6 to 3.25) and applies the operators there.
 constexpr int SJ = 16, SI = 4, SURF_THREADS = SJ * 3 * SI;
 struct SurfTile {
   float t1[3][SI + 4][3][SJ];   // xi traction, halo in x
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(256, 3) volume_interior_kernel(VolArgs a, int3
 }
 
 // Volume work of one stage: which box the tiled (or plain) interior kernel takes, the
-// units of the tiled PML kernel and the boxes of the general kernel.
+// units of the tiled PML kernel, the boxes of the general kernel and the free-surface rows.
 VolPlan plan_volume(const VolArgs& a, const TileCtx* tc) {
   const Dims& d = a.d;
   VolPlan pl;
@@ -555,7 +557,7 @@ static long long launch_flags(const VolArgs& a, cudaStream_t s, cudaStream_t s_s
   // directly behind the interior kernel unless timing events separate them
   if (pl.ps.nunits > 0) launch_pml(tc, a, FX, FY, FZ, bin, pl.ps, pl.pgrid, pl.tiled && !ke, s);
   if (fork && s_shell != s) {
-    // the general kernel on s_shell once the tiled kernels are done
+    // the kernels below on s_shell once the tiled ones are done
     cudaEventRecord(*fork, s);
     cudaStreamWaitEvent(s_shell, *fork, 0);
   }
@@ -597,8 +599,8 @@ void launch_shell_batch(const VolArgs* tab, const Boxes* boxes, const int* start
 }
 
 // Launches the volume kernels of one stage; kb/ke (optional) are recorded on s right
-// before and after the interior (tiled) kernel; with fork (and s_shell != s) the general
-// kernel runs on s_shell after the tiled kernels, else on s_shell right away.  Returns the
+// before and after the interior (tiled) kernel; with fork (and s_shell != s) the general and
+// free-surface kernels run on s_shell after the tiled kernels, else on s_shell right away.  Returns the
 // nodes of the box the interior kernel covers.
 long long launch_volume_stage(const VolArgs& a, int FX, int FY, int FZ, cudaStream_t s, cudaStream_t s_shell,
                               const TileCtx* tc, int bin, cudaEvent_t* kb, cudaEvent_t* ke, VolPlan* out,

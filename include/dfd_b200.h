@@ -301,8 +301,8 @@ int dfd_mlp_train(const float *x, const float *y, int n, int epochs, int batch, 
  *      which runs one job per process).  Every scenario is a context created, loaded and
  *      set up as usual on the same device; the ensemble advances all of them from step
  *      it0 with one batched launch per kernel and RK stage (fault node, fault band,
- *      general kernel) and one persistent launch of the tiled interior kernel whose units
- *      span every scenario, replayed from CUDA graphs.  Results stay in the scenarios'
+ *      free-surface rows) and one persistent launch each of the tiled interior and PML
+ *      kernels whose units span every scenario, replayed from CUDA graphs.  Results stay in the scenarios'
  *      contexts.  Destroy the ensemble before its contexts. ---- */
 typedef struct dfd_ens dfd_ens;
 int dfd_ens_create(dfd_ctx *const *scenarios, int n, dfd_ens **out);
