@@ -23,7 +23,10 @@ each of the four volume buffers (6.7 GB for the large domain) is far larger than
              nodes it updates, divided by its event-timed duration on its stream (an
              instrumented pass of up to 200 steps after the timed region, stages launched
              one by one with events around the kernel), against the measured HBM copy
-             bandwidth; volume_phase gives the same over all nodes and the volume phase
+             bandwidth; volume_phase gives the same over all nodes and the volume phase.
+             768 bytes are those of a scheme that stores its metric and keeps the RK
+             accumulator at every stage; the kernel moves fewer, so frac can pass 1.  moved
+             gives the rate of the DRAM bytes it does move (profiles/volume_traffic.json)
   cpu_baseline / --impl reference: the OpenMP FP32 CPU restatement of the same scheme
              (oracle/), the reference having no CPU path, on a bounded sample of steps
 
@@ -366,12 +369,12 @@ def run_ensemble(args, dfd, local):
     clocks = clk.stop()
     value = job_rate(nodes, args.steps, 1, ms / 1e3)
     nf = sum(p["NY"] * p["NZ"] for p, _, _ in specs)
-    # per step: 6 batched launches a stage (fault node, interior, PML, two groups of
-    # free-surface-row boxes, fault band), the rupture sensor of each rupture scenario,
-    # thermal pressurisation of each Friction_type 3 scenario, the step counter
+    # per step: 5 batched launches a stage (fault node, interior, PML, free-surface rows,
+    # fault band), the rupture sensor of each rupture scenario, thermal pressurisation of
+    # each Friction_type 3 scenario, the step counter
     n_rup = sum(1 for p, _, _ in specs if int(p.get("Rupture", 1)))
     n_tp = sum(1 for p, _, _ in specs if int(p.get("Rupture", 1)) and int(p.get("Friction_type", 0)) == 3)
-    ens_launches = 4 * 6 + n_rup + n_tp + 1
+    ens_launches = 4 * 5 + n_rup + n_tp + 1
     line = {"metric": "Gpt-steps/s", "value": value, "unit": "Gpt-steps/s", "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -538,6 +541,7 @@ def main():
     achieved = ALG_BYTES_PER_NODE_STEP * int_nodes * ksteps / (int_ms / 1e3) / 1e9
     phase = ALG_BYTES_PER_NODE_STEP * npts * ksteps / (vol_ms / 1e3) / 1e9
     tpn = traffic_per_node()
+    moved = tpn * int_nodes * ksteps / (int_ms / 1e3) / 1e9 if tpn else None
     line = {
         "metric": "Gpt-steps/s", "value": value, "unit": "Gpt-steps/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": max_ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -548,6 +552,7 @@ def main():
                      "traffic": tpn * int_nodes / 4 if tpn else None,
                      "kernel": "volume_tile_kernel (interior box, TMA-tiled)", "peak_source": peak_kind,
                      "bytes_per_node_step": ALG_BYTES_PER_NODE_STEP, "nodes_per_launch": int_nodes,
+                     "moved": {"bytes_per_node_step": tpn, "achieved": moved, "frac": moved / peak} if tpn else None,
                      "algorithmic_bytes_per_launch": ALG_BYTES_PER_NODE_STEP * int_nodes / 4,
                      "launch_us": 1e3 * int_ms / launches,
                      "timed": f"instrumented pass of {ksteps} steps after the timed region (per-kernel CUDA events, "
