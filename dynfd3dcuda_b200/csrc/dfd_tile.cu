@@ -21,15 +21,16 @@
 // 300 x 200, 18.5 M of them in the box) stages 0 to 3 went from 537 / 604 / 708 / 606 us to
 // 456 / 525 / 692 / 526 us, with 2 M nodes (200 x 100 x 100) from 43 / 48 / 57 / 47 to 40 /
 // 44 / 55 / 44 us.  Each stage has a bound of its own: a node needs 72 / 108 / 180 / 108
-// bytes and moves 78 / 126 / 205 / 126 in DRAM (stencil halo; 320 x 160 x 160 nodes), which at the times above is
-// 3.2 / 4.4 / 5.5 / 4.4 TB/s, and on 180 M nodes (3.24 / 3.76 / 5.21 / 3.76 ms) 3.5 / 4.9 /
-// 5.7 / 4.9 TB/s, where a copy reaches 6.46.  Only stage 2 is near memory.  The others wait:
-// 0.42 to 0.44 instructions issued per cycle and scheduler with 0.5 warps eligible of the two
-// that a scheduler has, their stalls on arithmetic, shared-memory and mbarrier latency.
+// bytes and moves 78 / 126 / 205 / 126 in DRAM (stencil halo; measured on 320 x 160 x 160
+// nodes).  At the times above that is 3.2 / 4.4 / 5.5 / 4.4 TB/s, and on 180 M nodes (3.24 /
+// 3.76 / 5.21 / 3.76 ms) 3.5 / 4.9 / 5.7 / 4.9 TB/s, where a copy reaches 6.46: only stage 2 is
+// near memory.  The others wait: 0.42 to 0.44 instructions issued per cycle and scheduler
+// with 0.5 warps eligible of the two that a scheduler has, their stalls on arithmetic,
+// shared-memory and mbarrier latency.
 //
-// The kernel is persistent: one CTA per SM (two with 4-row tiles) takes units (tile column x chunk) from a global
-// counter, and its copy stream runs across unit boundaries, so the next unit's planes
-// arrive while the current one finishes.
+// The kernel is persistent: one CTA per SM (two with 4-row tiles) takes units (tile column x
+// chunk) from a global counter, and its copy stream runs across unit boundaries, so the next
+// unit's planes arrive while the current one finishes.
 //
 // The right-hand side follows the reference's wave.cu:8-204 and rk4.cu:20-33, as the
 // kernels of dfd_volume.cu do.
